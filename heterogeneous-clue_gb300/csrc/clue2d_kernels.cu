@@ -348,6 +348,33 @@ __device__ __forceinline__ int next_chunk(int* s_next) {
   return __shfl_sync(0xffffffffu, base, 0);
 }
 
+// Running nearest higher over candidates in visiting order: the first
+// smallest d2 and, in `prev`, the smallest d2 before it.  The reference
+// compares sqrt_rn(d2) strictly, so the winner is the first candidate with the
+// smallest rounded square root: the one kept here unless a candidate visited
+// before it has a larger d2 with the same root.  Then `prev` is within the
+// margin of `d2`, near() is true and the query is decided again on square
+// roots.  A later candidate with an equal or larger d2 never replaces the
+// first.  Three moves under one predicate per candidate: a margin test on
+// each candidate instead (a product, a compare and the flag's logic) made
+// the search the larger part of the kernel (4096-event batch: 22.8 -> 20.5
+// ms, 200 HGCAL events: 6.30 -> 5.55 ms).
+struct NhBest {
+  float d2, prev;
+  int k = -1;
+  __device__ __forceinline__ explicit NhBest(float limit) : d2(limit), prev(limit) {}
+  __device__ __forceinline__ void visit(float2 pq, unsigned long long kq, const uint4& rk, int pos) {
+    const float d = dist2(pq, rec_xy(rk));
+    if (rec_key(rk) > kq && d < d2) {
+      prev = d2;
+      d2 = d;
+      k = pos;
+    }
+  }
+  // sqrt_rn(a) < sqrt_rn(b) whenever a * 1.00002f < b
+  __device__ __forceinline__ bool near() const { return !(__fmul_rn(d2, 1.00002f) < prev); }
+};
+
 // One (event, layer) item through every stage.  next_item: in thread 0, the
 // item this CTA takes next (-1 when none), whose inputs are prefetched.
 template <int NT, class TT, class QT>
@@ -495,11 +522,7 @@ __device__ void process_layer(const Params2D& P, const LayerStore<TT, QT>& S, co
   // "higher" (rho_j > rho_i, or equal rho and j > i) is key_j > key_i; a NaN
   // rho is higher than nothing and nothing is higher than it, as in the
   // reference.  The winner is the first candidate with the smallest
-  // correctly rounded sqrt(d2).  The loop keeps the first candidate with the
-  // smallest d2 and takes the exact sqrt comparison only for near ties:
-  //   d2 < 0.99999 * best_d2  implies  sqrt_rn(d2) < sqrt_rn(best_d2),
-  // so a candidate below `lim` always wins, one at or above best_d2 never
-  // does (sqrt_rn is monotone), and one in between is decided by sqrt_rn.
+  // correctly rounded sqrt(d2), found on d2 (NhBest).
   if (tid == 0) *s_next = 0;
   __syncthreads();
   int32_t* par = S.nh;  // parent: nearest higher for followers, -2 seed root, -3 other root
@@ -515,22 +538,12 @@ __device__ void process_layer(const Params2D& P, const LayerStore<TT, QT>& S, co
       const unsigned long long kq = rq.w == 0u ? ~0ull : ks;
       const int bx0 = tile_bin(__fsub_rn(pq.x, P.dm)), bx1 = tile_bin(__fadd_rn(pq.x, P.dm));
       const int by0 = tile_bin(__fsub_rn(pq.y, P.dm)), by1 = tile_bin(__fadd_rn(pq.y, P.dm));
-      float best_d2 = P.t_dm_next;  // d2 < t_dm_next <=> d2 <= t_dm
-      int best = -1;
-      bool near = false;
-      for_candidates(S.tbl, bx0, bx1, by0, by1, [&](int k) {
-        const uint4 rk = S.rec[k];
-        const float d2 = dist2(pq, rec_xy(rk));
-        const bool imp = (rec_key(rk) > kq) && d2 < best_d2;
-        // d2 * 1.00002 < best_d2 guarantees sqrt_rn(d2) < sqrt_rn(best_d2)
-        const bool win = imp && __fmul_rn(d2, 1.00002f) < best_d2;
-        near |= imp && !win;
-        best = win ? k : best;
-        best_d2 = win ? d2 : best_d2;
-      });
-      float best_s = best >= 0 ? __fsqrt_rn(best_d2) : FLT_MAX;
-      if (near) {
-        // a candidate came within the margin of the running best: decide this
+      NhBest nb(P.t_dm_next);  // d2 < t_dm_next <=> d2 <= t_dm
+      for_candidates(S.tbl, bx0, bx1, by0, by1, [&](int k) { nb.visit(pq, kq, S.rec[k], k); });
+      int best = nb.k;
+      float best_s = best >= 0 ? __fsqrt_rn(nb.d2) : FLT_MAX;
+      if (best >= 0 && nb.near()) {
+        // an earlier candidate's root may equal the winner's: decide this
         // query again with the reference's comparison on sqrt'd distances
         best_s = FLT_MAX;
         best = -1;
