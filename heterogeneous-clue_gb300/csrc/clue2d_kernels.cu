@@ -44,12 +44,28 @@
 #include <cstring>
 
 #include <algorithm>
+#include <utility>
 
 #include "clue_internal.h"
 
 namespace clue {
 
 namespace {
+
+// The kernels of one batch are launched with programmatic dependent launch:
+// each lets the next one's blocks onto the device as soon as all its own have
+// started (pdl_trigger) and waits for the whole previous kernel before it
+// touches memory (pdl_wait), so that a stage starts without a launch's
+// latency.  A kernel's completion implies its predecessors', since each waits
+// before it ends.  k_init, the first, is launched the ordinary way, and
+// k_label, the last, triggers nothing: work before and after a batch on the
+// stream sees ordinary kernels.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() {
+  pdl_wait();
+  pdl_trigger();
+}
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
@@ -615,16 +631,22 @@ __device__ void process_layer(const Params2D& P, const LayerStore<TT, QT>& S, co
 }
 // ------------------------------------------------------------------ kernels
 
-// Per-batch counters to their start values: layer counts and per-chunk seed
-// counts to 0, the tickets and pass counters to 0, "grouped" to 1 (k_count
-// clears it on the first layer decrease).  The error word is left alone: it
-// accumulates over the launches of a run.
+// Per-batch counters to their start values: layer counts, per-chunk seed
+// counts and size classes to 0, the tickets and pass counters to 0, "grouped"
+// to 1 (k_count clears it on the first layer decrease), and the error word to
+// 0 unless it accumulates over several batches (clear_error = 0).  It also
+// brings the batch's offset and chunk tables over from the host's page-locked
+// staging, so that a batch queues no copies and no memsets of its own: each of
+// those was a stream operation of 2-3 us, in a graph as well.
 __global__ void k_init(Batch2D b, int64_t n_lcnt) {
+  pdl_trigger();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < b.n_table_words) b.table_dst[i] = b.table_src[i];
   if (i < n_lcnt) b.lcnt[i] = 0;
   if (i < b.n_chunks) b.chunk_seeds[i] = 0;
-  if (i < kFlagCount - kFlagTicket) b.flags[kFlagTicket + i] = 0;
-  if (i == 0) b.flags[kFlagGrouped] = 1;
+  if (b.use_order && i < 2 * kSizeBuckets) b.size_hist[i] = 0;
+  if (i < kFlagCount && i != kFlagError) b.flags[i] = i == kFlagGrouped ? 1 : 0;
+  if (i == kFlagError && b.clear_error) b.flags[kFlagError] = 0;
 }
 
 __global__ void __launch_bounds__(kChunkThreads) k_count(Batch2D b) {
@@ -632,9 +654,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_count(Batch2D b) {
   __shared__ int s_e;
   __shared__ int s_cnt[kLayers];
   for (int l = threadIdx.x; l < kLayers; l += kChunkThreads) s_cnt[l] = 0;
-  // the size histogram of k_layer_scan starts from zero (it runs after this kernel)
-  if (c == 0 && b.use_order)
-    for (int i = threadIdx.x; i < 2 * kSizeBuckets; i += kChunkThreads) b.size_hist[i] = 0;
+  pdl_begin();
   if (threadIdx.x == 0) s_e = event_of_chunk(b, c);
   __syncthreads();
   const int e = s_e;
@@ -691,6 +711,7 @@ __device__ __forceinline__ int size_bucket(int m) { return kSizeBuckets - 1 - mi
 // One warp per event: layers 4*lane .. 4*lane+3.  Also counts the non-empty
 // layers per size class for k_order.
 __global__ void k_layer_scan(Batch2D b) {
+  pdl_begin();
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (e >= b.n_events) return;
   const int lane = lane_id();
@@ -735,6 +756,7 @@ __global__ void __launch_bounds__(kSizeBuckets) k_order(Batch2D b) {
   __shared__ int s_base[kSizeBuckets];
   __shared__ int s_ws[33];
   const int tid = threadIdx.x;
+  pdl_begin();
   const int v = b.size_hist[tid];
   int total;
   const int inc = block_inclusive_scan<kSizeBuckets>(v, s_ws, &total);
@@ -759,6 +781,7 @@ __global__ void __launch_bounds__(kSizeBuckets) k_order(Batch2D b) {
 }
 
 __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
+  pdl_begin();
   if (b.flags[kFlagGrouped]) return;  // input already grouped by layer
   const int c = blockIdx.x;
   __shared__ int s_e;
@@ -804,6 +827,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_layers(Batch2D b, Params2D P,
   __shared__ int s_next;
   __shared__ int s_ws[33];
   __shared__ int s_bins[64];
+  pdl_begin();
   const int n_items = b.use_order ? b.flags[kFlagOrdered] : b.n_events * kLayers;
   const bool grouped = b.flags[kFlagGrouped] != 0;
   LayerStore<uint16_t, uint16_t> sm;
@@ -873,6 +897,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_layers(Batch2D b, Params2D P,
 }
 // One warp per event: exclusive scan of its chunks' seed counts.
 __global__ void k_seed_chunk_scan(Batch2D b) {
+  pdl_begin();
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (e >= b.n_events) return;
   const int lane = lane_id();
@@ -898,6 +923,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_seed_rank(Batch2D b) {
   const int c = blockIdx.x;
   __shared__ int s_e;
   __shared__ int s_ws[33];
+  pdl_begin();
   if (threadIdx.x == 0) s_e = event_of_chunk(b, c);
   __syncthreads();
   const int e = s_e;
@@ -925,6 +951,9 @@ __global__ void __launch_bounds__(kChunkThreads) k_seed_rank(Batch2D b) {
 __global__ void __launch_bounds__(kChunkThreads) k_label(Batch2D b) {
   const int c = blockIdx.x;
   __shared__ int s_e;
+  pdl_wait();
+  // the run's status words, final by now, to the host's page-locked copy
+  if (c == 0 && threadIdx.x < kFlagCount && b.host_flags) b.host_flags[threadIdx.x] = b.flags[threadIdx.x];
   if (threadIdx.x == 0) s_e = event_of_chunk(b, c);
   __syncthreads();
   const int e = s_e;
@@ -957,13 +986,29 @@ __global__ void __launch_bounds__(kChunkThreads) k_label(Batch2D b) {
   }
 }
 
+// Queues a kernel that begins with pdl_wait().
+template <class... Params, class... Args>
+cudaError_t launch_pdl(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                       Args&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 template <int NT>
 cudaError_t launch_layers(const Batch2D& b, const Params2D& p, int cap, int max_m, int big_pass, int grid,
                           cudaStream_t s) {
   Tuning2D t;
   t.layer_capacity = cap;
-  k_layers<NT><<<grid, NT, layer_smem_bytes(t), s>>>(b, p, cap, max_m, big_pass);
-  return cudaGetLastError();
+  return launch_pdl(k_layers<NT>, grid, NT, layer_smem_bytes(t), s, b, p, cap, max_m, big_pass);
 }
 
 cudaError_t launch_layers_any(int threads, const Batch2D& b, const Params2D& p, int cap, int max_m, int big_pass,
@@ -1107,29 +1152,28 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
     // counters, tickets and flags of this batch (seeds per chunk are counted
     // by k_layers as it flags them)
     const int64_t n_lcnt = (int64_t)b.n_events * kLayers;
-    const int64_t n_init = std::max<int64_t>(std::max<int64_t>(n_lcnt, nc), kFlagCount);
+    const int64_t n_init = std::max({n_lcnt, (int64_t)nc, b.n_table_words, (int64_t)2 * kSizeBuckets});
     NvtxRange r("clue2d/init");
     k_init<<<(unsigned)((n_init + 255) / 256), 256, 0, s>>>(b, n_lcnt);
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
   }
   const int warps_grid = (b.n_events * 32 + 255) / 256;
   mark(0);
   {
     NvtxRange r("clue2d/count");
-    k_count<<<nc, kChunkThreads, 0, s>>>(b);
+    if ((err = launch_pdl(k_count, nc, kChunkThreads, 0, s, b)) != cudaSuccess) return err;
   }
   mark(1);
   {
     NvtxRange r("clue2d/layer_scan");
-    k_layer_scan<<<warps_grid, 256, 0, s>>>(b);
-    if (b.use_order) k_order<<<warps_grid, kSizeBuckets, 0, s>>>(b);
+    if ((err = launch_pdl(k_layer_scan, warps_grid, 256, 0, s, b)) != cudaSuccess) return err;
+    if (b.use_order && (err = launch_pdl(k_order, warps_grid, kSizeBuckets, 0, s, b)) != cudaSuccess) return err;
   }
   mark(2);
   {
     NvtxRange r("clue2d/scatter");
-    k_scatter<<<nc, kChunkThreads, 0, s>>>(b);
+    if ((err = launch_pdl(k_scatter, nc, kChunkThreads, 0, s, b)) != cudaSuccess) return err;
   }
-  err = cudaGetLastError();
-  if (err != cudaSuccess) return err;
   mark(3);
   const int n_items = b.n_events * kLayers;
   // No more layers than SMs (a single event): one pass of the widest CTA per
@@ -1168,21 +1212,21 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
   mark(4);
   {
     NvtxRange r("clue2d/seed_chunk_scan");
-    k_seed_chunk_scan<<<warps_grid, 256, 0, s>>>(b);
+    if ((err = launch_pdl(k_seed_chunk_scan, warps_grid, 256, 0, s, b)) != cudaSuccess) return err;
   }
   mark(5);
   {
     NvtxRange r("clue2d/seed_rank");
-    k_seed_rank<<<nc, kChunkThreads, 0, s>>>(b);
+    if ((err = launch_pdl(k_seed_rank, nc, kChunkThreads, 0, s, b)) != cudaSuccess) return err;
   }
   mark(6);
   {
     NvtxRange r("clue2d/label");
-    k_label<<<nc, kChunkThreads, 0, s>>>(b);
+    if ((err = launch_pdl(k_label, nc, kChunkThreads, 0, s, b)) != cudaSuccess) return err;
   }
   mark(7);
   if (kernels) *kernels += 8 + (b.use_order ? 1 : 0) + (two_class ? 1 : 0);
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 }  // namespace clue

@@ -76,6 +76,13 @@ struct Batch2D {
   int32_t n_events = 0;
   int64_t n_points = 0;
   int32_t n_chunks = 0;
+  // offset and chunk tables in page-locked host memory, copied word by word to
+  // table_dst by the first kernel (0 words: the tables are on the device)
+  const int32_t* table_src = nullptr;
+  int32_t* table_dst = nullptr;
+  int64_t n_table_words = 0;
+  int32_t clear_error = 1;        // 0: the error word accumulates over batches
+  int32_t* host_flags = nullptr;  // page-locked copy of `flags`, written by the last kernel (nullptr: none)
   const int64_t* offsets = nullptr;      // [E+1]
   const int32_t* chunk_start = nullptr;  // [E+1] first chunk of each event
   const int32_t* chunk_ev = nullptr;     // [n_chunks] event of each chunk (nullptr: searched in chunk_start)

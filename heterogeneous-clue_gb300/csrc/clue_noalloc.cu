@@ -154,8 +154,6 @@ extern "C" int clue_run_event_noalloc(const clue_params* params, int32_t n, cons
 
   k_noalloc_event_header<<<1, 1, 0, s>>>(const_cast<int64_t*>(b.offsets), const_cast<int32_t*>(b.chunk_start), n);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "launching CLUE kernels");
-  if ((e = cudaMemsetAsync(b.flags + kFlagError, 0, sizeof(int32_t), s)) != cudaSuccess)
-    return cuda_error(e, "clearing status");
   if ((e = launch_clue2d(b, p, t, s)) != cudaSuccess) return cuda_error(e, "launching CLUE kernels");
   int32_t err_word = 0;
   if ((e = cudaMemcpyAsync(&err_word, b.flags + kFlagError, sizeof(int32_t), cudaMemcpyDeviceToHost, s)) !=

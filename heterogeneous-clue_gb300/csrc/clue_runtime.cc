@@ -126,9 +126,10 @@ int PinnedBuf::reserve(size_t n) {
 namespace {
 
 enum Slot2D : int {
-  S_OFF, S_CS, S_LCNT, S_LSTART, S_CURSOR, S_GX, S_GY, S_GW, S_GID,
+  S_TABLES,  // offsets | chunk_start | chunk_ev, back to back as in the pinned staging
+  S_LCNT, S_LSTART, S_CURSOR, S_GX, S_GY, S_GW, S_GID,
   S_SP0, S_SP1, S_SP2, S_SP3, S_SP4, S_SP5, S_SP6, S_SP7,
-  S_SPTBL, S_CSEED, S_CBASE, S_FLAGS, S_ORDER, S_CEV,
+  S_SPTBL, S_CSEED, S_CBASE, S_FLAGS, S_ORDER,
   S_IN,   // host runs: x | y | layer | w of the run, each N long, back to back
   S_OUT,  // host runs: rho | delta | nearestHigher | isSeed | clusterIndex, likewise
   S_COUNT
@@ -140,10 +141,13 @@ int64_t n_chunks_of(int32_t n_events, const int64_t* off) {
   return c;
 }
 
+// Bytes of the offset and chunk tables of a batch: offsets (8 B each), the
+// first chunk of each event, the event of each chunk.
+size_t table_bytes(int32_t E, int64_t nchunks) { return 12 * (size_t)(E + 1) + 4 * (size_t)nchunks; }
+
 std::vector<size_t> sizes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bool host_io) {
   std::vector<size_t> s(S_COUNT, 0);
-  s[S_OFF] = 8 * (size_t)(E + 1);
-  s[S_CS] = 4 * (size_t)(E + 1);
+  s[S_TABLES] = table_bytes(E, nchunks);
   s[S_LCNT] = s[S_LSTART] = s[S_CURSOR] = 4 * (size_t)E * kLayers;
   s[S_GX] = s[S_GY] = s[S_GW] = s[S_GID] = 4 * (size_t)N;
   // spill homes: 16-byte records, then nh and the query order (4 B each)
@@ -151,7 +155,7 @@ std::vector<size_t> sizes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bo
   s[S_SP1] = s[S_SP2] = s[S_SP3] = s[S_SP6] = s[S_SP7] = 0;
   s[S_SP4] = s[S_SP5] = 4 * (size_t)N;
   s[S_SPTBL] = 4 * (size_t)kTableStride * grid;
-  s[S_CSEED] = s[S_CBASE] = s[S_CEV] = 4 * (size_t)std::max<int64_t>(nchunks, 1);
+  s[S_CSEED] = s[S_CBASE] = 4 * (size_t)std::max<int64_t>(nchunks, 1);
   s[S_FLAGS] = 4 * kFlagCount;
   s[S_ORDER] = 4 * ((size_t)E * kLayers + 2 * kSizeBuckets);
   if (host_io) {
@@ -252,16 +256,6 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
   cudaStream_t s = h->stream;
   cudaError_t e;
   const size_t n4 = 4 * (size_t)r.N;
-  e = cudaMemsetAsync(b.flags + kFlagError, 0, 4, s);
-  if (e != cudaSuccess) return cuda_error(e, "clearing status");
-  e = cudaMemcpyAsync((void*)b.offsets, h->stage.p, 8 * (size_t)(r.E + 1), cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return cuda_error(e, "H2D offsets");
-  e = cudaMemcpyAsync((void*)b.chunk_start, static_cast<char*>(h->stage.p) + 8 * (size_t)(r.E + 1),
-                      4 * (size_t)(r.E + 1), cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return cuda_error(e, "H2D chunk table");
-  e = cudaMemcpyAsync((void*)b.chunk_ev, static_cast<char*>(h->stage.p) + 12 * (size_t)(r.E + 1),
-                      4 * (size_t)b.n_chunks, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return cuda_error(e, "H2D chunk events");
   if (host_io) {
     // back-to-back host arrays (a server's staging) move in one copy
     const char* hx = reinterpret_cast<const char*>(r.x);
@@ -295,8 +289,6 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
       return cuda_error(e, "D2H outputs");
     }
   }
-  e = cudaMemcpyAsync(h->flags_host.p, b.flags, 4 * kFlagCount, cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) return cuda_error(e, "D2H status");
   return CLUE_OK;
 }
 
@@ -316,15 +308,22 @@ void host_io_views(void* in, void* out, int64_t N, Batch2D& b) {
   b.ci = reinterpret_cast<int32_t*>(fo + 4 * N);
 }
 
-void fill_batch_views(Handle* h, const Run2D& r, int64_t nchunks, bool host_io, Batch2D& b,
-                      const DeviceArena* arena = nullptr) {
+// `tables`: the batch's tables in the pinned staging, `flags`: the pinned copy
+// of its status words.
+void fill_batch_views(Handle* h, const Run2D& r, int64_t nchunks, bool host_io, Batch2D& b, const void* tables,
+                      int32_t* flags, const DeviceArena* arena = nullptr) {
   const DeviceArena& A = arena ? *arena : h->arena;
   auto P = [&](int slot) { return A.ptr(slot); };
   b.n_events = r.E;
   b.n_points = r.N;
   b.n_chunks = (int32_t)nchunks;
-  b.offsets = static_cast<const int64_t*>(P(S_OFF));
-  b.chunk_start = static_cast<const int32_t*>(P(S_CS));
+  b.table_src = static_cast<const int32_t*>(tables);
+  b.table_dst = static_cast<int32_t*>(P(S_TABLES));
+  b.n_table_words = tables ? (int64_t)(table_bytes(r.E, nchunks) / 4) : 0;
+  b.offsets = static_cast<const int64_t*>(P(S_TABLES));
+  b.chunk_start = b.table_dst + 2 * (size_t)(r.E + 1);
+  b.chunk_ev = b.chunk_start + (r.E + 1);
+  b.host_flags = flags;
   if (host_io) {
     host_io_views(P(S_IN), P(S_OUT), r.N, b);
   } else {
@@ -349,7 +348,6 @@ void fill_batch_views(Handle* h, const Run2D& r, int64_t nchunks, bool host_io, 
   b.sp_tbl = static_cast<int32_t*>(P(S_SPTBL));
   b.chunk_seeds = static_cast<int32_t*>(P(S_CSEED));
   b.chunk_base = static_cast<int32_t*>(P(S_CBASE));
-  b.chunk_ev = static_cast<const int32_t*>(P(S_CEV));
   b.flags = static_cast<int32_t*>(P(S_FLAGS));
   b.order = static_cast<int32_t*>(P(S_ORDER));
   b.size_hist = b.order + (size_t)r.E * kLayers;
@@ -379,7 +377,7 @@ int run_2d_batched(Handle* h, const Run2D& r, cudaEvent_t* stage_events = nullpt
   if (rc) return rc;
 
   Batch2D b;
-  fill_batch_views(h, r, nchunks, host_io, b);
+  fill_batch_views(h, r, nchunks, host_io, b, h->stage.p, static_cast<int32_t*>(h->flags_host.p));
 
   bool use_graph = !(r.flags & CLUE_NO_GRAPH) && !stage_events;
   if (use_graph && host_io) {
@@ -398,7 +396,7 @@ int run_2d_batched(Handle* h, const Run2D& r, cudaEvent_t* stage_events = nullpt
                  h->tuning.work_tile_cm, h->p2d.dc, h->p2d.rhoc, h->p2d.odf,
                  {(const void*)r.x, (const void*)r.y, (const void*)r.layer, (const void*)r.w,
                   (const void*)r.out->rho, (const void*)r.out->delta, (const void*)r.out->nearestHigher,
-                  (const void*)r.out->isSeed, (const void*)r.out->clusterIndex, h->arena.ptr(S_OFF),
+                  (const void*)r.out->isSeed, (const void*)r.out->clusterIndex, h->arena.ptr(S_TABLES),
                   h->arena.ptr(S_GX), h->arena.ptr(S_SP0), h->stage.p, h->flags_host.p}};
     // A graph pays off when a shape repeats (the same event sizes, buffers and
     // tuning): a run whose key differs from the previous run's goes by direct
@@ -475,8 +473,7 @@ int run_2d_plain(Handle* h, const Run2D& r) {
     need[S_IN] = 16 * (size_t)maxn;
     need[S_OUT] = 20 * (size_t)maxn;
   }
-  need[S_OFF] = 16 * (size_t)std::max(r.E, 1);
-  need[S_CS] = 8 * (size_t)std::max(r.E, 1);
+  need[S_TABLES] = 24 * (size_t)std::max(r.E, 1);  // the offsets of every event, then their chunk tables
   rc = h->arena.reserve(need, h->budget);
   if (rc) return rc;
   rc = h->stage.reserve(24 * (size_t)std::max(r.E, 1));
@@ -494,10 +491,8 @@ int run_2d_plain(Handle* h, const Run2D& r) {
   cudaStream_t s = h->stream;
   cudaError_t e = cudaMemsetAsync(h->arena.ptr(S_FLAGS), 0, 4 * kFlagCount, s);
   if (e != cudaSuccess) return cuda_error(e, "clearing status");
-  e = cudaMemcpyAsync(h->arena.ptr(S_OFF), so, 16 * (size_t)r.E, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return cuda_error(e, "H2D offsets");
-  e = cudaMemcpyAsync(h->arena.ptr(S_CS), sc, 8 * (size_t)r.E, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return cuda_error(e, "H2D chunk table");
+  e = cudaMemcpyAsync(h->arena.ptr(S_TABLES), so, 24 * (size_t)r.E, cudaMemcpyHostToDevice, s);
+  if (e != cudaSuccess) return cuda_error(e, "H2D offset and chunk tables");
   int any_error = 0;
   h->last_run.h2d_bytes = 24 * (int64_t)r.E + (host_io ? 16 * r.N : 0);
   h->last_run.d2h_bytes = 0;
@@ -509,10 +504,11 @@ int run_2d_plain(Handle* h, const Run2D& r) {
     one.E = 1;
     one.N = n;
     Batch2D b;
-    fill_batch_views(h, one, sc[2 * ev + 1], false, b);
+    fill_batch_views(h, one, sc[2 * ev + 1], false, b, nullptr, nullptr);
     b.chunk_ev = nullptr;  // one event: every chunk is event 0
-    b.offsets = static_cast<const int64_t*>(h->arena.ptr(S_OFF)) + 2 * ev;
-    b.chunk_start = static_cast<const int32_t*>(h->arena.ptr(S_CS)) + 2 * ev;
+    b.clear_error = 0;     // accumulates over the events
+    b.offsets = static_cast<const int64_t*>(h->arena.ptr(S_TABLES)) + 2 * ev;
+    b.chunk_start = static_cast<const int32_t*>(h->arena.ptr(S_TABLES)) + 4 * (size_t)r.E + 2 * ev;
     const size_t n4 = 4 * (size_t)n;
     if (host_io) {
       host_io_views(h->arena.ptr(S_IN), h->arena.ptr(S_OUT), n, b);
@@ -570,9 +566,9 @@ int run_2d_plain(Handle* h, const Run2D& r) {
 // into sub-batches of about kPipePoints points that take turns on
 // kPipeSlots device slots.  Three streams overlap the H2D copy of one sub-batch, the
 // kernels of the previous one and the D2H copy of the one before that:
-//   in-copy  : wait comp[k] (slot inputs free)  -> offsets, chunk table, x, y, layer, w -> h2d[k]
+//   in-copy  : wait comp[k] (slot inputs free)  -> x, y, layer, w -> h2d[k]
 //   compute  : wait h2d[k], d2h[k] (slot outputs free) -> kernels -> comp[k]
-//   out-copy : wait comp[k] -> rho, delta, nh, isSeed, clusterIndex, status -> d2h[k]
+//   out-copy : wait comp[k] -> rho, delta, nh, isSeed, clusterIndex -> d2h[k]
 // Sub-batches hold whole events, so every output is the one of the
 // unsplit batch.
 constexpr int64_t kPipePoints = int64_t(8) << 20;
@@ -638,6 +634,7 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
   int64_t kernels = 0;
   for (int i = 0; i < S; ++i) {
     const int k = i % kPipeSlots;
+    fh[kFlagCount * (size_t)i + kFlagError] = 0;  // a sub-batch of empty events launches nothing
     const int32_t e0 = cut[i], Es = cut[i + 1] - e0;
     const int64_t p0 = r.off[e0], Ns = r.off[cut[i + 1]] - p0;
     // staging: rebased offsets, then the chunk table
@@ -655,17 +652,12 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
     sub.N = Ns;
     sub.off = so;
     Batch2D b;
-    fill_batch_views(h, sub, sc[Es], true, b, slot_arena[k]);
+    fill_batch_views(h, sub, sc[Es], true, b, so, fh + kFlagCount * (size_t)i, slot_arena[k]);
     const size_t n4 = 4 * (size_t)Ns;
     // kernels of both slots stay on the handle's stream: letting the next
     // sub-batch's persistent kernel start beside the draining one measured slower
     cudaStream_t ci = h->copy_in, co = h->copy_out, cs = h->stream;
     if ((e = cudaStreamWaitEvent(ci, comp[k], 0)) != cudaSuccess ||
-        (e = cudaMemcpyAsync((void*)b.offsets, so, 8 * (size_t)(Es + 1), cudaMemcpyHostToDevice, ci)) != cudaSuccess ||
-        (e = cudaMemcpyAsync((void*)b.chunk_start, sc, 4 * (size_t)(Es + 1), cudaMemcpyHostToDevice, ci)) !=
-            cudaSuccess ||
-        (e = cudaMemcpyAsync((void*)b.chunk_ev, sce, 4 * (size_t)sc[Es], cudaMemcpyHostToDevice, ci)) !=
-            cudaSuccess ||
         (e = cudaMemcpyAsync((void*)b.x, r.x + p0, n4, cudaMemcpyHostToDevice, ci)) != cudaSuccess ||
         (e = cudaMemcpyAsync((void*)b.y, r.y + p0, n4, cudaMemcpyHostToDevice, ci)) != cudaSuccess ||
         (e = cudaMemcpyAsync((void*)b.layer, r.layer + p0, n4, cudaMemcpyHostToDevice, ci)) != cudaSuccess ||
@@ -673,8 +665,7 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
         (e = cudaEventRecord(h2d[k], ci)) != cudaSuccess)
       return cuda_error(e, "H2D sub-batch");
     if ((e = cudaStreamWaitEvent(cs, h2d[k], 0)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(cs, d2h[k], 0)) != cudaSuccess ||
-        (e = cudaMemsetAsync(b.flags + kFlagError, 0, 4, cs)) != cudaSuccess)
+        (e = cudaStreamWaitEvent(cs, d2h[k], 0)) != cudaSuccess)
       return cuda_error(e, "sub-batch set-up");
     if ((e = launch_clue2d(b, h->p2d, h->tuning, cs, nullptr, &kernels)) != cudaSuccess)
       return cuda_error(e, "launching CLUE kernels");
@@ -686,8 +677,6 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
         (e = cudaMemcpyAsync(o->nearestHigher + p0, b.nh, n4, cudaMemcpyDeviceToHost, co)) != cudaSuccess ||
         (e = cudaMemcpyAsync(o->isSeed + p0, b.seed, n4, cudaMemcpyDeviceToHost, co)) != cudaSuccess ||
         (e = cudaMemcpyAsync(o->clusterIndex + p0, b.ci, n4, cudaMemcpyDeviceToHost, co)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(fh + kFlagCount * (size_t)i, b.flags, 4 * kFlagCount, cudaMemcpyDeviceToHost, co)) !=
-            cudaSuccess ||
         (e = cudaEventRecord(d2h[k], co)) != cudaSuccess)
       return cuda_error(e, "D2H sub-batch");
   }
