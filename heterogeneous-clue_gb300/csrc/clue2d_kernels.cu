@@ -780,31 +780,52 @@ __global__ void __launch_bounds__(kSizeBuckets) k_order(Batch2D b) {
   }
 }
 
+// Each chunk's points to their layers' grouped positions: counted per layer in
+// shared memory first, so that a block reserves its places with one global
+// atomic per layer (the order inside a layer is arbitrary: k_layers restores
+// the index order).  With a global atomic per warp group of every pass the
+// passes ran one after another at its round trip: 57 -> 21 us on one shuffled
+// HGCAL event of 323k points.
 __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
-  pdl_begin();
-  if (b.flags[kFlagGrouped]) return;  // input already grouped by layer
   const int c = blockIdx.x;
   __shared__ int s_e;
+  __shared__ int s_cnt[kLayers];  // the block's points per layer, then the position of the first
+  for (int l = threadIdx.x; l < kLayers; l += kChunkThreads) s_cnt[l] = 0;
+  pdl_begin();
+  if (b.flags[kFlagGrouped]) return;  // input already grouped by layer
   if (threadIdx.x == 0) s_e = event_of_chunk(b, c);
   __syncthreads();
   const int e = s_e;
   const int64_t es = b.offsets[e], ee = b.offsets[e + 1];
   const int64_t i0 = es + (int64_t)(c - b.chunk_start[e]) * kChunk;
   const int64_t i1 = min(i0 + (int64_t)kChunk, ee);
-  const unsigned lt = (1u << lane_id()) - 1u;
-  for (int64_t base = i0; base < i1; base += kChunkThreads) {
-    const int64_t i = base + threadIdx.x;
-    int key = -1;
-    if (i < i1) {
-      const int l = b.layer[i];
-      if (l >= 0 && l < kLayers) key = e * kLayers + l;
-    }
-    const unsigned mask = __match_any_sync(0xffffffffu, key);
+  const int lane = lane_id();
+  const unsigned lt = (1u << lane) - 1u;
+  constexpr int PER = kChunk / kChunkThreads;
+  int lv[PER], rank[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
+    lv[j] = i < i1 ? b.layer[i] : -1;
+    if (lv[j] >= kLayers) lv[j] = -1;
+  }
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const unsigned mask = __match_any_sync(0xffffffffu, lv[j]);
     const int leader = __ffs(mask) - 1;
-    int pos = 0;
-    if (key >= 0 && lane_id() == leader) pos = atomicAdd(&b.cursor[key], __popc(mask));
-    pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(mask & lt);
-    if (key >= 0) {
+    int old = 0;
+    if (lv[j] >= 0 && lane == leader) old = atomicAdd(&s_cnt[lv[j]], __popc(mask));
+    rank[j] = __shfl_sync(0xffffffffu, old, leader) + __popc(mask & lt);
+  }
+  __syncthreads();
+  for (int l = threadIdx.x; l < kLayers; l += kChunkThreads)
+    if (s_cnt[l]) s_cnt[l] = atomicAdd(&b.cursor[e * kLayers + l], s_cnt[l]);
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
+    if (lv[j] >= 0) {
+      const int pos = s_cnt[lv[j]] + rank[j];
       b.gx[pos] = b.x[i];
       b.gy[pos] = b.y[i];
       b.gw[pos] = b.w[i];
