@@ -191,6 +191,8 @@ struct Batch3D {
   int32_t* flags = nullptr;    // [kFlagCount]
 };
 
+// Opts the CLUE3D search kernels into the shared memory they use, on the current device.
+cudaError_t prepare_clue3d_kernels();
 cudaError_t launch_clue3d(const Batch3D& b, const Params3D& p, cudaStream_t s);
 
 }  // namespace clue

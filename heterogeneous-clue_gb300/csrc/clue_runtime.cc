@@ -770,6 +770,7 @@ int clue_create(const clue_params* params, size_t budget, int device, void* stre
     e = cudaSetDevice(device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
     e = clue::prepare_clue2d_kernels(device);
+    if (e == cudaSuccess) e = clue::prepare_clue3d_kernels();
     if (e != cudaSuccess) return cuda_error(e, "preparing kernels");
     Handle* h = new Handle();
     h->device = device;
