@@ -44,28 +44,13 @@
 #include <cstring>
 
 #include <algorithm>
-#include <utility>
 
 #include "clue_internal.h"
+#include "clue_pdl.cuh"
 
 namespace clue {
 
 namespace {
-
-// The kernels of one batch are launched with programmatic dependent launch:
-// each lets the next one's blocks onto the device as soon as all its own have
-// started (pdl_trigger) and waits for the whole previous kernel before it
-// touches memory (pdl_wait), so that a stage starts without a launch's
-// latency.  A kernel's completion implies its predecessors', since each waits
-// before it ends.  k_init, the first, is launched the ordinary way, and
-// k_label, the last, triggers nothing: work before and after a batch on the
-// stream sees ordinary kernels.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_begin() {
-  pdl_wait();
-  pdl_trigger();
-}
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
@@ -641,6 +626,7 @@ __global__ void k_init(Batch2D b, int64_t n_lcnt) {
   pdl_trigger();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < b.n_table_words) b.table_dst[i] = b.table_src[i];
+  if (i < b.n_in16) b.in_dst[i] = b.host_in[i];
   if (i < n_lcnt) b.lcnt[i] = 0;
   if (i < b.n_chunks) b.chunk_seeds[i] = 0;
   if (b.use_order && i < 2 * kSizeBuckets) b.size_hist[i] = 0;
@@ -1004,23 +990,20 @@ __global__ void __launch_bounds__(kChunkThreads) k_label(Batch2D b) {
     const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
     if (i < i1 && v[j] <= -2) b.ci[i] = r[j];
   }
-}
-
-// Queues a kernel that begins with pdl_wait().
-template <class... Params, class... Args>
-cudaError_t launch_pdl(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                       Args&&... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  if (b.host_out) {  // a small host run's outputs, array after array
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
+      if (i < i1) {
+        float* o = b.host_out + i;
+        o[0] = b.rho[i];
+        o[b.n_points] = b.delta[i];
+        o[2 * b.n_points] = __int_as_float(b.nh[i]);
+        o[3 * b.n_points] = __int_as_float(b.seed[i]);
+        o[4 * b.n_points] = __int_as_float(v[j] <= -2 ? r[j] : v[j]);
+      }
+    }
+  }
 }
 
 template <int NT>
@@ -1172,7 +1155,7 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
     // counters, tickets and flags of this batch (seeds per chunk are counted
     // by k_layers as it flags them)
     const int64_t n_lcnt = (int64_t)b.n_events * kLayers;
-    const int64_t n_init = std::max({n_lcnt, (int64_t)nc, b.n_table_words, (int64_t)2 * kSizeBuckets});
+    const int64_t n_init = std::max({n_lcnt, (int64_t)nc, b.n_table_words, b.n_in16, (int64_t)2 * kSizeBuckets});
     NvtxRange r("clue2d/init");
     k_init<<<(unsigned)((n_init + 255) / 256), 256, 0, s>>>(b, n_lcnt);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;

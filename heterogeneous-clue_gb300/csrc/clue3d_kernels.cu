@@ -12,6 +12,7 @@
 // arcs in the reference's order.
 //
 // Stages (one launch each, flattened over all events of the batch):
+//   k3_init       counters and masks to zero, tables over from the host
 //   k3_key        flat key per cluster; clusters per (event, row) and each
 //                 cluster's arrival slot in its row
 //   k3_row_scan   per event: first position of each row
@@ -23,16 +24,18 @@
 //                     (event, slab of layers) with the slab's rows staged
 //   k3_search<false>  KernelComputeDistanceToHigherSoA (:286-392), likewise,
 //                     then seeds, outliers and parent pointers (:509-560)
-//   k3_finish     per event: trackster ids by seed rank, pointer jumping
-//                 along nearestHigher, labels (:564-577)
+//   k3_finish     per event: trackster ids by seed rank, walks along
+//                 nearestHigher, labels (:564-577)
 // Float arithmetic uses explicit _rn intrinsics in the reference's operation
 // order; phiBin's product is in double, as in TICLLayerTile.h:28-34.
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cmath>
 #include <cstdint>
 
 #include "clue_internal.h"
+#include "clue_pdl.cuh"
 
 namespace clue {
 namespace {
@@ -67,10 +70,22 @@ __device__ __forceinline__ int eta_bin(float eta, const Params3D& P) {
 // A NaN (phi NaN or +-inf, which reduce to NaN) takes bin 0: the reference's
 // int conversion is undefined there, 0 on the aarch64 host, and the device's
 // conversion would give INT_MIN.
+__device__ __noinline__ int phi_bin_double(float norm, float phi_r) {
+  if (norm != norm) return 0;
+  return __double2int_rz(__dmul_rn(__dadd_rn((double)norm, 3.14159265358979323846), (double)phi_r));
+}
+
+// The same bin from the single-precision product where that cannot lie on the
+// other side of a bin edge: the sum is off by at most 3.3e-7 (the float pi, one
+// rounding below 6.3), times 20.05 bins per radian, plus half an ulp of 126:
+// 1.1e-5, so values 1e-4 and more from an edge truncate alike; the others
+// (one in 5,000) call the double form.
 __device__ __forceinline__ int phi_bin(float phi, const Params3D& P) {
   const float norm = reduce_range(phi, P);
-  if (norm != norm) return 0;
-  return __double2int_rz(__dmul_rn(__dadd_rn((double)norm, 3.14159265358979323846), (double)P.phi_r));
+  const float t = __fmul_rn(__fadd_rn(norm, P.pi_f), P.phi_r);
+  const float f = t - truncf(t);
+  if (t > 0.f && t < 127.f && f > 1e-4f && f < 1.f - 1e-4f) return __float2int_rz(t);
+  return phi_bin_double(norm, P.phi_r);
 }
 
 // The reference's layer window (CLUE3DAlgoKernels.h:49-58 density, :308-317
@@ -93,7 +108,28 @@ __device__ __forceinline__ void layer_window(int layer, int sib, int n_layers, i
 // event's last row, which no search visits.
 __device__ __forceinline__ int row_of(int k, int n_rows) { return k >= 0 ? k / kPhiBins : n_rows - 1; }
 
+// Row counts, row masks and status words to zero, the offset and block tables
+// (and a small host run's inputs) over from the host's page-locked staging: a
+// run queues kernels only.
+__global__ void k3_init(Batch3D b) {
+  pdl_trigger();
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = i0; i < b.n_table_words; i += step) b.table_dst[i] = b.table_src[i];
+  for (int64_t i = i0; i < b.n_in16; i += step) b.in_dst[i] = b.host_in[i];
+  const int64_t rows = (int64_t)b.n_events * b.n_rows;
+  uint4* m = reinterpret_cast<uint4*>(b.row_mask);
+  uint4* r = reinterpret_cast<uint4*>(b.row_rep);
+  for (int64_t i = i0; i < rows; i += step) {
+    b.row_cnt[i] = 0;
+    m[i] = make_uint4(0u, 0u, 0u, 0u);
+    r[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (i0 < kFlagCount) b.flags[i0] = 0;
+}
+
 __global__ void k3_key(Batch3D b, Params3D P) {
+  pdl_begin();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int row = -1, e = 0;
   if (i < b.n_points) {
@@ -133,6 +169,7 @@ __device__ __forceinline__ int bits_below(unsigned long long m0, unsigned long l
 
 // One block per event: exclusive scan of its rows.
 __global__ void __launch_bounds__(256) k3_row_scan(Batch3D b) {
+  pdl_begin();
   const int e = blockIdx.x;
   const int R = b.n_rows;
   const int per = (R + 255) / 256;
@@ -168,6 +205,7 @@ __global__ void __launch_bounds__(256) k3_row_scan(Batch3D b) {
 // The cluster also goes into its row's 128-bit phi-column occupancy mask;
 // bit 127 marks a column held twice.
 __global__ void k3_scatter(Batch3D b, Params3D P) {
+  pdl_begin();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= b.n_points) return;
   const int e = event_of_blk(b, i);
@@ -209,6 +247,7 @@ __global__ void k3_scatter(Batch3D b, Params3D P) {
 // repeats, a count over the row otherwise.  One thread per scattered entry;
 // its records move within the row's range.
 __global__ void k3_row_sort(Batch3D b) {
+  pdl_begin();
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= b.n_points) return;
   const int e = event_of_blk(b, p);
@@ -627,6 +666,7 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
   int32_t* s_rs = reinterpret_cast<int32_t*>(s_rep + 4 * kSlabMaxRows);
   uint32_t* s_before = reinterpret_cast<uint32_t*>(s_rs + kSlabMaxRows + 1);
   uint8_t* s_col = reinterpret_cast<uint8_t*>(s_before + kSlabMaxRows + 1);
+  pdl_begin();
   const int e = blockIdx.x / n_slabs;
   const int L0 = (blockIdx.x % n_slabs) * kSlabLayers;
   const int L1 = min(L0 + kSlabLayers, P.n_layers);
@@ -740,66 +780,93 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
 }
 
 
-// One block per event: trackster ids by seed rank in index order, then
-// pointer jumping along nearestHigher (replaces the LIFO propagation), then
-// labels.  par holds event-local indices.
-__global__ void __launch_bounds__(512) k3_finish(Batch3D b) {
+// One block per event: trackster ids by seed rank in index order, then each
+// cluster's walk along nearestHigher to its root and its label (replaces the
+// LIFO propagation).  par holds event-local indices.  Eight clusters per
+// thread and scan round, and one walk instead of rounds of pointer jumping
+// over the event: 20 -> XX us on one event of 5,000 clusters (a launch of one
+// block), 0.153 -> XX ms on 1,000 events.
+constexpr int kFinishThreads = 512;
+constexpr int kFinishPer = 8;
+
+__global__ void __launch_bounds__(kFinishThreads) k3_finish(Batch3D b) {
+  pdl_wait();
   const int e = blockIdx.x;
   const int64_t es = b.offsets[e];
   const int n = (int)(b.offsets[e + 1] - es);
   int32_t* par = b.par + es;
   int32_t* ti = b.ti + es;
   int32_t* seed = b.seed + es;
-  __shared__ int s_w[16];
-  __shared__ int s_base;
+  __shared__ int s_w[kFinishThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_base = 0;
-  __syncthreads();
-  for (int base = 0; base < n; base += 512) {
-    const int i = base + threadIdx.x;
-    int f = (i < n) ? seed[i] : 0;
-    if (f < 0) {  // rejected by k3_key: no seed, a root of its own
-      f = 0;
-      seed[i] = 0;
-      par[i] = -3;
+  int base_rank = 0;
+  for (int base = 0; base < n; base += kFinishThreads * kFinishPer) {
+    const int i0 = base + threadIdx.x * kFinishPer;
+    int f[kFinishPer], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kFinishPer; ++j) f[j] = i0 + j < n ? seed[i0 + j] : 0;
+#pragma unroll
+    for (int j = 0; j < kFinishPer; ++j) {
+      if (f[j] < 0) {  // rejected by k3_key: no seed, a root of its own
+        f[j] = 0;
+        seed[i0 + j] = 0;
+        par[i0 + j] = -3;
+      }
+      sum += f[j];
     }
-    int x = f;
+    int x = sum;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += t;
     }
     if (lane == 31) s_w[warp] = x;
     __syncthreads();
-    int before = s_base;
-    for (int w = 0; w < warp; ++w) before += s_w[w];
-    if (i < n) ti[i] = f ? before + x - 1 : -1;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int tot = 0;
-      for (int w = 0; w < 16; ++w) tot += s_w[w];
-      s_base += tot;
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kFinishThreads / 32; ++w) {
+      if (w < warp) before += s_w[w];
+      total += s_w[w];
     }
+    int rank = base_rank + before + x - sum;
+#pragma unroll
+    for (int j = 0; j < kFinishPer; ++j)
+      if (f[j]) ti[i0 + j] = rank++;
+    base_rank += total;
     __syncthreads();
   }
-  if (threadIdx.x == 0) b.ev_seeds[e] = s_base;
+  if (threadIdx.x == 0) {
+    b.ev_seeds[e] = base_rank;
+    if (b.host_nt) b.host_nt[e] = base_rank;
+  }
+  if (e == 0 && threadIdx.x < kFlagCount && b.host_flags) b.host_flags[threadIdx.x] = b.flags[threadIdx.x];
+  // walks of 64 steps without a root leave their pointer at the farthest
+  // cluster reached and are taken up again in another pass
   for (;;) {
-    int changed = 0;
-    for (int i = threadIdx.x; i < n; i += 512) {
-      const int p = par[i];
-      if (p >= 0) {
-        const int pp = par[p];
-        if (pp >= 0) {
-          par[i] = pp;
-          changed = 1;
-        }
+    int unresolved = 0;
+    for (int i = threadIdx.x; i < n; i += kFinishThreads) {
+      int r = i, p = par[i];
+      if (p == -2) continue;  // a seed: labelled above
+      for (int step = 0; p >= 0 && step < 64; ++step) {
+        r = p;
+        p = par[r];
+      }
+      if (p < 0) {
+        ti[i] = p == -2 ? ti[r] : -1;
+      } else {
+        par[i] = r;
+        unresolved = 1;
       }
     }
-    if (!__syncthreads_or(changed)) break;
+    if (!__syncthreads_or(unresolved)) break;
   }
-  for (int i = threadIdx.x; i < n; i += 512) {
-    if (seed[i]) continue;
-    const int p = par[i];
-    ti[i] = (p >= 0 && par[p] == -2) ? ti[p] : -1;
+  if (b.host_out) {  // a small host run's outputs, array after array
+    const float* o[7] = {b.rho, b.delta_t, reinterpret_cast<const float*>(b.delta_l),
+                         reinterpret_cast<const float*>(b.nh_l), reinterpret_cast<const float*>(b.nh_i),
+                         reinterpret_cast<const float*>(b.seed), reinterpret_cast<const float*>(b.ti)};
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+      for (int i = threadIdx.x; i < n; i += kFinishThreads) b.host_out[k * b.n_points + es + i] = o[k][es + i];
   }
 }
 
@@ -814,46 +881,50 @@ cudaError_t prepare_clue3d_kernels() {
 
 cudaError_t launch_clue3d(const Batch3D& b, const Params3D& p, cudaStream_t s) {
   if (b.n_events <= 0 || b.n_points <= 0) return cudaSuccess;
-  cudaError_t err = cudaMemsetAsync(b.row_cnt, 0, sizeof(int32_t) * (size_t)b.n_events * b.n_rows, s);
-  if (err != cudaSuccess) return err;
-  err = cudaMemsetAsync(b.row_mask, 0, 16 * (size_t)b.n_events * b.n_rows, s);
-  if (err != cudaSuccess) return err;
-  err = cudaMemsetAsync(b.row_rep, 0, 16 * (size_t)b.n_events * b.n_rows, s);
-  if (err != cudaSuccess) return err;
+  cudaError_t err;
   const int T = 256;
   const int grid = (int)((b.n_points + T - 1) / T);
   {
+    NvtxRange r("clue3d/init");
+    const int64_t work = std::max({(int64_t)b.n_events * b.n_rows, b.n_table_words, b.n_in16});
+    k3_init<<<(unsigned)std::min<int64_t>((work + T - 1) / T, 8192), T, 0, s>>>(b);
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
+  }
+  {
     NvtxRange r("clue3d/key");
-    k3_key<<<grid, T, 0, s>>>(b, p);
+    if ((err = launch_pdl(k3_key, grid, T, 0, s, b, p)) != cudaSuccess) return err;
   }
   {
     NvtxRange r("clue3d/row_scan");
-    k3_row_scan<<<b.n_events, 256, 0, s>>>(b);
+    if ((err = launch_pdl(k3_row_scan, b.n_events, 256, 0, s, b)) != cudaSuccess) return err;
   }
   {
     NvtxRange r("clue3d/scatter");
-    k3_scatter<<<grid, T, 0, s>>>(b, p);
+    if ((err = launch_pdl(k3_scatter, grid, T, 0, s, b, p)) != cudaSuccess) return err;
   }
   {
     NvtxRange r("clue3d/row_sort");
-    k3_row_sort<<<grid, T, 0, s>>>(b);
+    if ((err = launch_pdl(k3_row_sort, grid, T, 0, s, b)) != cudaSuccess) return err;
   }
   const int n_slabs = (p.n_layers + kSlabLayers - 1) / kSlabLayers;
   const int64_t slab_blocks = (int64_t)b.n_events * n_slabs;
   if (slab_blocks > INT32_MAX) return cudaErrorInvalidValue;
   {
     NvtxRange r("clue3d/density");
-    k3_search<true><<<(unsigned)slab_blocks, kSlabThreads, kSlabSmem, s>>>(b, p, n_slabs);
+    if ((err = launch_pdl(k3_search<true>, (unsigned)slab_blocks, kSlabThreads, kSlabSmem, s, b, p, n_slabs)) != cudaSuccess)
+      return err;
   }
   {
     NvtxRange r("clue3d/nearest_higher");
-    k3_search<false><<<(unsigned)slab_blocks, kSlabThreads, kSlabSmem, s>>>(b, p, n_slabs);
+    if ((err = launch_pdl(k3_search<false>, (unsigned)slab_blocks, kSlabThreads, kSlabSmem, s, b, p, n_slabs)) !=
+        cudaSuccess)
+      return err;
   }
   {
     NvtxRange r("clue3d/finish");
-    k3_finish<<<b.n_events, 512, 0, s>>>(b);
+    if ((err = launch_pdl(k3_finish, b.n_events, kFinishThreads, 0, s, b)) != cudaSuccess) return err;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 }  // namespace clue

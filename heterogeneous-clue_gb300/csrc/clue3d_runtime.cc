@@ -45,9 +45,11 @@ Params3D make_params3d(const clue3d_params& q) {
 }
 
 enum Slot3D : int {
-  T_OFF, T_BEV, T_KEY, T_RCNT, T_RSTART, T_ARR, T_SORTED, T_SCOL, T_TMP, T_PAR, T_EVSEEDS, T_FLAGS, T_MASK, T_REP, T_CAND, T_QREC, T_TCAND, T_TQREC,
-  T_IN0, T_IN1, T_IN2, T_IN3, T_IN4, T_IN5, T_IN6, T_IN7,
-  T_OUT0, T_OUT1, T_OUT2, T_OUT3, T_OUT4, T_OUT5, T_OUT6,
+  T_TABLES,  // event offsets | event of each 256-cluster block, as in the pinned staging
+  T_KEY, T_RCNT, T_RSTART, T_ARR, T_SORTED, T_SCOL, T_TMP, T_PAR, T_EVSEEDS, T_FLAGS, T_MASK, T_REP, T_CAND, T_QREC,
+  T_TCAND, T_TQREC,
+  T_IN,   // host runs: the 8 inputs, each N long, back to back
+  T_OUT,  // host runs: the 7 outputs, likewise
   T_COUNT
 };
 
@@ -110,9 +112,9 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     if (rc) return rc;
     const bool host_io = !(flags & CLUE_DEVICE_MEMORY);
     std::vector<size_t> need(T_COUNT, 0);
-    need[T_OFF] = 8 * (size_t)(E + 1);
     const int64_t n_blk = (N + 255) / 256;
-    need[T_BEV] = 4 * (size_t)n_blk;
+    const size_t table_bytes = 8 * (size_t)(E + 1) + 4 * (size_t)n_blk;
+    need[T_TABLES] = table_bytes;
     need[T_KEY] = need[T_ARR] = need[T_SORTED] = need[T_SCOL] = need[T_TMP] = need[T_PAR] = 4 * (size_t)N;
     need[T_RCNT] = 4 * (size_t)(E * n_rows);
     need[T_RSTART] = 4 * (size_t)(E * n_rows + 1);
@@ -121,16 +123,22 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     need[T_MASK] = need[T_REP] = 16 * (size_t)(E * n_rows);
     need[T_CAND] = need[T_QREC] = need[T_TCAND] = need[T_TQREC] = 16 * (size_t)N;
     if (host_io) {
-      for (int s = T_IN0; s <= T_OUT6; ++s) need[s] = 4 * (size_t)N;
+      need[T_IN] = 32 * (size_t)N;
+      need[T_OUT] = 28 * (size_t)N;
     }
     rc = h->arena3d.reserve(need, h->budget > h->arena.total() ? h->budget - h->arena.total() : 0);
     if (rc) return rc;
-    rc = h->stage.reserve(8 * (size_t)(E + 1) + 4 * (size_t)n_blk);
+    rc = h->stage.reserve(table_bytes);
     if (rc) return rc;
     rc = h->flags_host.reserve(4 * kFlagCount);
     if (rc) return rc;
     rc = h->nt_host.reserve(4 * (size_t)E);
     if (rc) return rc;
+    const bool staged = host_io && N <= kStagedIoPoints && host_accessible(ins, 8) && host_accessible(outs, 7);
+    if (staged) {
+      rc = h->io_stage.reserve(60 * (size_t)N);
+      if (rc) return rc;
+    }
     memcpy(h->stage.p, off, 8 * (size_t)(E + 1));
     // the event of each 256-cluster block's first cluster, so that a kernel
     // finds a cluster's event in a step or two instead of a binary search
@@ -146,25 +154,32 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     b.n_events = E;
     b.n_points = N;
     b.n_rows = (int32_t)n_rows;
-    b.offsets = static_cast<const int64_t*>(P(T_OFF));
+    b.table_src = static_cast<const int32_t*>(h->stage.p);
+    b.table_dst = static_cast<int32_t*>(P(T_TABLES));
+    b.n_table_words = (int64_t)(table_bytes / 4);
+    b.host_nt = static_cast<int32_t*>(h->nt_host.p);
+    b.host_flags = static_cast<int32_t*>(h->flags_host.p);
+    b.offsets = static_cast<const int64_t*>(P(T_TABLES));
+    b.blk_ev = b.table_dst + 2 * (size_t)(E + 1);
     const void* din[8];
     void* dout[7];
     const size_t n4 = 4 * (size_t)N;
-    if ((e = cudaMemsetAsync(P(T_FLAGS), 0, 4 * kFlagCount, s)) != cudaSuccess) return cuda_error(e, "memset");
-    if ((e = cudaMemcpyAsync(P(T_OFF), h->stage.p, 8 * (size_t)(E + 1), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(P(T_BEV), bev, 4 * (size_t)n_blk, cudaMemcpyHostToDevice, s)) != cudaSuccess)
-      return cuda_error(e, "H2D offsets");
-    b.blk_ev = static_cast<const int32_t*>(P(T_BEV));
     for (int i = 0; i < 8; ++i) {
-      if (host_io) {
-        din[i] = P(T_IN0 + i);
-        if ((e = cudaMemcpyAsync(P(T_IN0 + i), ins[i], n4, cudaMemcpyHostToDevice, s)) != cudaSuccess)
+      din[i] = host_io ? static_cast<char*>(P(T_IN)) + i * n4 : ins[i];
+      if (staged) {
+        memcpy(static_cast<char*>(h->io_stage.p) + i * n4, ins[i], n4);
+      } else if (host_io) {
+        if ((e = cudaMemcpyAsync(const_cast<void*>(din[i]), ins[i], n4, cudaMemcpyHostToDevice, s)) != cudaSuccess)
           return cuda_error(e, "H2D layer clusters");
-      } else {
-        din[i] = ins[i];
       }
     }
-    for (int i = 0; i < 7; ++i) dout[i] = host_io ? P(T_OUT0 + i) : outs[i];
+    for (int i = 0; i < 7; ++i) dout[i] = host_io ? static_cast<char*>(P(T_OUT)) + i * n4 : outs[i];
+    if (staged) {
+      b.host_in = static_cast<const uint4*>(h->io_stage.p);
+      b.in_dst = static_cast<uint4*>(P(T_IN));
+      b.n_in16 = 2 * N;  // 8 arrays of 4 N bytes
+      b.host_out = reinterpret_cast<float*>(static_cast<char*>(h->io_stage.p) + 8 * n4);
+    }
     b.z = static_cast<const float*>(din[0]);
     b.eta = static_cast<const float*>(din[1]);
     b.phi = static_cast<const float*>(din[2]);
@@ -198,20 +213,19 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     b.tqrec = static_cast<float4*>(P(T_TQREC));
     e = launch_clue3d(b, make_params3d(*prm), s);
     if (e != cudaSuccess) return cuda_error(e, "launching CLUE3D kernels");
-    if (host_io) {
+    if (host_io && !staged) {
       for (int i = 0; i < 7; ++i)
         if ((e = cudaMemcpyAsync(outs[i], dout[i], n4, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
           return cuda_error(e, "D2H outputs");
     }
-    if ((e = cudaMemcpyAsync(h->nt_host.p, b.ev_seeds, 4 * (size_t)E, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(h->flags_host.p, b.flags, 4 * kFlagCount, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-      return cuda_error(e, "D2H status");
     if ((e = cudaEventRecord(h->done_event, s)) != cudaSuccess) return cuda_error(e, "cudaEventRecord");
     h->pending = true;
     h->error_layers = prm->n_layers;
     if (host_io) {
       rc = h->wait_previous();
       if (rc) return rc;
+      if (staged)
+        for (int i = 0; i < 7; ++i) memcpy(outs[i], static_cast<char*>(h->io_stage.p) + (8 + i) * n4, n4);
       const int32_t* f = static_cast<const int32_t*>(h->flags_host.p);
       if (f[kFlagError] == 2) {
         static_cast<int32_t*>(h->flags_host.p)[kFlagError] = 0;

@@ -82,6 +82,12 @@ struct Batch2D {
   int32_t* table_dst = nullptr;
   int64_t n_table_words = 0;
   int32_t clear_error = 1;        // 0: the error word accumulates over batches
+  // a small host run: its inputs (n_in16 x 16 bytes, copied to in_dst) and its
+  // outputs (5 arrays of n_points) in page-locked host memory
+  const uint4* host_in = nullptr;
+  uint4* in_dst = nullptr;
+  int64_t n_in16 = 0;
+  float* host_out = nullptr;
   int32_t* host_flags = nullptr;  // page-locked copy of `flags`, written by the last kernel (nullptr: none)
   const int64_t* offsets = nullptr;      // [E+1]
   const int32_t* chunk_start = nullptr;  // [E+1] first chunk of each event
@@ -155,6 +161,19 @@ struct Batch3D {
   int32_t n_events = 0;
   int64_t n_points = 0;
   int32_t n_rows = 0;  // rows (layer, eta) per event: n_layers * 34 + 1
+  // page-locked host memory the kernels read and write: the offset and block
+  // tables (copied to table_dst), the trackster counts and status words
+  // (nullptr: none), and of a small host run its inputs (n_in16 x 16 bytes,
+  // copied to in_dst) and outputs (7 arrays of n_points; nullptr: none)
+  const int32_t* table_src = nullptr;
+  int32_t* table_dst = nullptr;
+  int64_t n_table_words = 0;
+  int32_t* host_nt = nullptr;
+  int32_t* host_flags = nullptr;
+  const uint4* host_in = nullptr;
+  uint4* in_dst = nullptr;
+  int64_t n_in16 = 0;
+  float* host_out = nullptr;
   const int64_t* offsets = nullptr;  // [E+1]
   const int32_t* blk_ev = nullptr;   // [ceil(N / 256)] event of each 256-cluster block's first cluster
   const float* z = nullptr;

@@ -176,6 +176,18 @@ bool is_pinned_or_device(const void* p) {
 
 }  // namespace
 
+bool host_accessible(const void* const* p, int n) {
+  for (int i = 0; i < n; ++i) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p[i]) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type == cudaMemoryTypeDevice) return false;
+  }
+  return true;
+}
+
 size_t required_bytes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bool host_io) {
   auto s = sizes_2d(E, N, nchunks, grid, host_io);
   size_t t = 0;
@@ -256,7 +268,7 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
   cudaStream_t s = h->stream;
   cudaError_t e;
   const size_t n4 = 4 * (size_t)r.N;
-  if (host_io) {
+  if (host_io && !b.host_in) {
     // back-to-back host arrays (a server's staging) move in one copy
     const char* hx = reinterpret_cast<const char*>(r.x);
     if (reinterpret_cast<const char*>(r.y) == hx + n4 && reinterpret_cast<const char*>(r.layer) == hx + 2 * n4 &&
@@ -272,7 +284,7 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
   }
   e = launch_clue2d(b, h->p2d, h->tuning, s, stage_events, kernels);
   if (e != cudaSuccess) return cuda_error(e, "launching CLUE kernels");
-  if (host_io) {
+  if (host_io && !b.host_out) {
     const clue_outputs* o = r.out;
     const char* ho = reinterpret_cast<const char*>(o->rho);
     if (reinterpret_cast<const char*>(o->delta) == ho + n4 &&
@@ -353,10 +365,31 @@ void fill_batch_views(Handle* h, const Run2D& r, int64_t nchunks, bool host_io, 
   b.size_hist = b.order + (size_t)r.E * kLayers;
 }
 
-int run_2d_batched(Handle* h, const Run2D& r, cudaEvent_t* stage_events = nullptr) {
+int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nullptr) {
+  Run2D r = r_in;
   const bool host_io = !(r.flags & CLUE_DEVICE_MEMORY);
   int rc = h->wait_previous();
   if (rc) return rc;
+  // a small host run: through page-locked staging, inputs back to back, then outputs
+  const void* io[9] = {r.x, r.y, r.layer, r.w, r.out->rho, r.out->delta, r.out->nearestHigher, r.out->isSeed,
+                       r.out->clusterIndex};
+  const bool staged = host_io && !(r.flags & kAsyncHostIO) && r.N <= kStagedIoPoints && host_accessible(io, 9);
+  clue_outputs staged_out;
+  if (staged) {
+    const size_t n4 = 4 * (size_t)r.N;
+    rc = h->io_stage.reserve(9 * n4);
+    if (rc) return rc;
+    char* st = static_cast<char*>(h->io_stage.p);
+    for (int i = 0; i < 4; ++i) memcpy(st + i * n4, io[i], n4);
+    r.x = reinterpret_cast<const float*>(st);
+    r.y = reinterpret_cast<const float*>(st + n4);
+    r.layer = reinterpret_cast<const int32_t*>(st + 2 * n4);
+    r.w = reinterpret_cast<const float*>(st + 3 * n4);
+    staged_out = clue_outputs{reinterpret_cast<float*>(st + 4 * n4), reinterpret_cast<float*>(st + 5 * n4),
+                              reinterpret_cast<int32_t*>(st + 6 * n4), reinterpret_cast<int32_t*>(st + 7 * n4),
+                              reinterpret_cast<int32_t*>(st + 8 * n4)};
+    r.out = &staged_out;
+  }
   const int64_t nchunks = n_chunks_of(r.E, r.off);
   const int grid = layer_grid_max(h->tuning, std::max(1, r.E * kLayers));
   rc = h->arena.reserve(sizes_2d(r.E, r.N, nchunks, grid, host_io), h->budget);
@@ -379,8 +412,15 @@ int run_2d_batched(Handle* h, const Run2D& r, cudaEvent_t* stage_events = nullpt
   Batch2D b;
   fill_batch_views(h, r, nchunks, host_io, b, h->stage.p, static_cast<int32_t*>(h->flags_host.p));
 
+  if (staged) {
+    b.host_in = reinterpret_cast<const uint4*>(r.x);
+    b.in_dst = reinterpret_cast<uint4*>(const_cast<float*>(b.x));
+    b.n_in16 = r.N;  // 4 arrays of 4 N bytes
+    b.host_out = r.out->rho;
+  }
+
   bool use_graph = !(r.flags & CLUE_NO_GRAPH) && !stage_events;
-  if (use_graph && host_io) {
+  if (use_graph && host_io && !staged) {
     // graph memcpy nodes need page-locked host memory
     use_graph = is_pinned_or_device(r.x) && is_pinned_or_device(r.y) && is_pinned_or_device(r.layer) &&
                 is_pinned_or_device(r.w) && is_pinned_or_device(r.out->rho) &&
@@ -454,6 +494,9 @@ int run_2d_batched(Handle* h, const Run2D& r, cudaEvent_t* stage_events = nullpt
   if (host_io && !(r.flags & kAsyncHostIO)) {
     rc = h->wait_previous();
     if (rc) return rc;
+    if (staged)
+      for (int i = 4; i < 9; ++i)
+        memcpy(const_cast<void*>(io[i]), static_cast<char*>(h->io_stage.p) + 4 * (size_t)r.N * i, 4 * (size_t)r.N);
     return h->check_device_flags();
   }
   return CLUE_OK;

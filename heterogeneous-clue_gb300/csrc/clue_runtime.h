@@ -100,6 +100,16 @@ size_t arena_bytes_after_2d(const Handle* h, int32_t E, int64_t N, int64_t nchun
 // queued; completion is seen through Handle::done_event.  Used by the server.
 constexpr int kAsyncHostIO = 0x100;
 
+// Host-memory runs of up to this many points (or layer clusters) go through
+// page-locked staging that the first kernel reads and the last one writes: two
+// host copies instead of a stream copy per array (9 or 15 of them, each
+// staged by the driver).  Producer call on 5k / 25k points 105 -> 64 / 143 ->
+// 105 us; at 50k points the host copies cost more (152 -> 163 us).  CLUE3D on
+// 5k layer clusters 168 -> 118 us, on 50k 252 -> 300 us.
+constexpr int64_t kStagedIoPoints = int64_t(32) << 10;
+// Whether the CPU may read and write all of these arrays.
+bool host_accessible(const void* const* p, int n);
+
 // Device slots of the pipelined host-memory path (sub-batches in flight).
 constexpr int kPipeSlots = 2;
 
@@ -125,6 +135,7 @@ struct Handle {
   PinnedBuf stage;
   PinnedBuf flags_host;
   PinnedBuf nt_host;
+  PinnedBuf io_stage;  // inputs and outputs of small host-memory runs
   cudaGraphExec_t graph_exec = nullptr;
   GraphKey graph_key;
   GraphKey last_key;  // the previous graph-eligible run (a shape is captured when it repeats)
