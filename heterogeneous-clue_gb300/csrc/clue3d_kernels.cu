@@ -24,7 +24,7 @@
 //                     (event, slab of layers) with the slab's rows staged
 //   k3_search<false>  KernelComputeDistanceToHigherSoA (:286-392), likewise,
 //                     then seeds, outliers and parent pointers (:509-560)
-//   k3_finish     per event: trackster ids by seed rank, walks along
+//   k3_rank, k3_label   trackster ids by seed rank, walks along
 //                 nearestHigher, labels (:564-577)
 // Float arithmetic uses explicit _rn intrinsics in the reference's operation
 // order; phiBin's product is in double, as in TICLLayerTile.h:28-34.
@@ -107,6 +107,34 @@ __device__ __forceinline__ void layer_window(int layer, int sib, int n_layers, i
 // Row of a flat key; clusters rejected by k3_key (key -1) go to the
 // event's last row, which no search visits.
 __device__ __forceinline__ int row_of(int k, int n_rows) { return k >= 0 ? k / kPhiBins : n_rows - 1; }
+
+// A placed cluster is one 32-byte record, a whole memory sector written by one
+// store: as a candidate {roa, phi, energy, rho} (rho added by the density
+// search), as a query {z, event-local index, density threshold, bins}.  Records
+// go to scattered places; in pieces (two 16-byte records, the index and the
+// column in arrays of their own) half the sectors reached DRAM partly written
+// and were read back to be completed.
+__device__ __forceinline__ void store_record(float4* rec, int64_t at, float roa, float phi, float energy, float z, int idx,
+                                             float thr, int bins) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(rec + 2 * at), "r"(__float_as_int(roa)),
+               "r"(__float_as_int(phi)), "r"(__float_as_int(energy)), "r"(0), "r"(__float_as_int(z)), "r"(idx),
+               "r"(__float_as_int(thr)), "r"(bins)
+               : "memory");
+}
+
+// bins: layer | etaBin << 11 | phiBin << 17 | isSilicon << 24, or -1 for a
+// cluster rejected by the binning (its row is never searched).
+__device__ __forceinline__ int pack_bins(int l, int eb, int pb, bool sil) {
+  return l | (eb << 11) | (pb << 17) | ((sil ? 1 : 0) << 24);
+}
+__device__ __forceinline__ int bins_key(int bins) {
+  return (bins & 0x7ff) * kBins + ((bins >> 17) & 0x7f) + ((bins >> 11) & 0x3f) * kPhiBins;
+}
+// Phi column in the row: phi bin 126 is column 0 of the next row.
+__device__ __forceinline__ int bins_col(int bins) {
+  const int pb = (bins >> 17) & 0x7f;
+  return pb < kPhiBins ? pb : 0;
+}
 
 // Row counts, row masks and status words to zero, the offset and block tables
 // (and a small host run's inputs) over from the host's page-locked staging: a
@@ -196,14 +224,9 @@ __global__ void __launch_bounds__(256) k3_row_scan(Batch3D b) {
   if (e == b.n_events - 1 && threadIdx.x == 255) b.row_start[(int64_t)b.n_events * R] = (int)b.offsets[b.n_events];
 }
 
-// Each cluster to its arrival slot in its row, with everything the row sort
-// and the searches need of it, read here in input order (coalesced): its
-// event-local index, phi column and row; its 16-byte candidate record {roa,
-// phi, energy, rho} (rho added by the density search); its 16-byte query
-// record {z, roa * z, density threshold, layer | etaBin << 11 | phiBin << 17 |
-// isSilicon << 24}.
-// The cluster also goes into its row's 128-bit phi-column occupancy mask;
-// bit 127 marks a column held twice.
+// Each cluster's record, read here in input order (coalesced), to its arrival
+// slot in its row.  The cluster also goes into its row's 128-bit phi-column
+// occupancy mask; bit 127 marks a column held twice.
 __global__ void k3_scatter(Batch3D b, Params3D P) {
   pdl_begin();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -213,23 +236,19 @@ __global__ void k3_scatter(Batch3D b, Params3D P) {
   const int row = row_of(k, b.n_rows);
   const int64_t r = (int64_t)e * b.n_rows + row;
   const int pos = b.row_start[r] + b.arr[i];
-  const int col = k >= 0 ? k % kPhiBins : 0;
-  b.tmp[pos] = (int32_t)(i - b.offsets[e]);
-  b.par[pos] = col | (row << 7);
-  const float roa = b.roa[i];
-  b.tcand[pos] = make_float4(roa, b.phi[i], b.energy[i], 0.f);
-  if (k >= 0) {
-    const float zi = b.z[i];
-    const float thr = b.sil[i] ? P.dens_thr : __fmul_rn(b.radius[i], b.radius[i]);
-    // the phi bin from the key (key = layer * 4284 + phiBin + 126 * etaBin,
-    // phiBin up to 126), without k3_key's double-precision product again
-    const int li = b.layer[i], eb = eta_bin(b.eta[i], P);
-    const int pbin = k - li * kBins - eb * kPhiBins;
-    const int bins = li | (eb << 11) | (pbin << 17) | ((b.sil[i] ? 1 : 0) << 24);
-    b.tqrec[pos] = make_float4(zi, __fmul_rn(roa, zi), thr, __int_as_float(bins));
-  } else {
-    b.tqrec[pos] = make_float4(0.f, 0.f, 0.f, 0.f);  // the junk row's entries are never queried
+  const int idx = (int)(i - b.offsets[e]);
+  if (k < 0) {  // the last row's entries are never queried
+    store_record(b.trec, pos, 0.f, 0.f, 0.f, 0.f, idx, 0.f, -1);
+    return;
   }
+  // the phi bin from the key (key = layer * 4284 + phiBin + 126 * etaBin,
+  // phiBin up to 126)
+  const int li = b.layer[i], eb = eta_bin(b.eta[i], P);
+  const bool sil = b.sil[i];
+  const float radius = b.radius[i];
+  store_record(b.trec, pos, b.roa[i], b.phi[i], b.energy[i], b.z[i], idx, sil ? P.dens_thr : __fmul_rn(radius, radius),
+               pack_bins(li, eb, k - li * kBins - eb * kPhiBins, sil));
+  const int col = k % kPhiBins;
   unsigned long long* m = b.row_mask + 2 * r;
   const unsigned long long bit = 1ull << (col & 63);
   if (atomicOr(m + (col >> 6), bit) & bit) {
@@ -245,15 +264,17 @@ __global__ void k3_scatter(Batch3D b, Params3D P) {
 // a counting sort by column through the occupancy mask (the entries in lower
 // columns are the mask's set bits below the entry's column) when no column
 // repeats, a count over the row otherwise.  One thread per scattered entry;
-// its records move within the row's range.
+// its record moves within the row's range.
 __global__ void k3_row_sort(Batch3D b) {
   pdl_begin();
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= b.n_points) return;
+  const float4 c = b.trec[2 * p], d = b.trec[2 * p + 1];
+  const int bins = __float_as_int(d.w), idx = __float_as_int(d.y);
+  if (bins < 0) return;
   const int e = event_of_blk(b, p);
-  const int idx = b.tmp[p], cr = b.par[p];
-  const int col = cr & 127;
-  const int64_t r = (int64_t)e * b.n_rows + (cr >> 7);
+  const int col = bins_col(bins);
+  const int64_t r = (int64_t)e * b.n_rows + bins_key(bins) / kPhiBins;
   const int s = b.row_start[r];
   const ulonglong2 m = reinterpret_cast<const ulonglong2*>(b.row_mask)[r];
   int rank;
@@ -263,15 +284,12 @@ __global__ void k3_row_sort(Batch3D b) {
     const int t = b.row_start[r + 1];
     rank = 0;
     for (int q = s; q < t; ++q) {
-      const int c2 = b.par[q] & 127, i2 = b.tmp[q];
+      const float4 o = b.trec[2 * (int64_t)q + 1];
+      const int c2 = bins_col(__float_as_int(o.w)), i2 = __float_as_int(o.y);
       rank += (c2 < col) || (c2 == col && i2 < idx);
     }
   }
-  const int f = s + rank;
-  b.sorted[f] = idx;
-  b.scol[f] = col;
-  b.cand[f] = b.tcand[p];
-  b.qrec[f] = b.tqrec[p];
+  store_record(b.rec, s + rank, c.x, c.y, c.z, d.x, idx, d.z, bins);
 }
 
 // The rows of one event as the searches see them: the whole event in global
@@ -280,13 +298,12 @@ __global__ void k3_row_sort(Batch3D b) {
 struct RowsGlobal {
   const unsigned long long* mask;  // 2 words per row of the event
   const int32_t* rstart;           // first sorted position of each row of the event
-  const float4* cand;
-  const int32_t* scol;
+  const float4* recs;              // 2 per entry
   __device__ __forceinline__ unsigned long long m0(int r) const { return mask[2 * r]; }
   __device__ __forceinline__ unsigned long long m1(int r) const { return mask[2 * r + 1]; }
   __device__ __forceinline__ int start(int r) const { return rstart[r]; }
-  __device__ __forceinline__ float4 rec(int q) const { return cand[q]; }
-  __device__ __forceinline__ int col(int q) const { return scol[q]; }
+  __device__ __forceinline__ float4 rec(int q) const { return recs[2 * (int64_t)q]; }
+  __device__ __forceinline__ int col(int q) const { return bins_col(__float_as_int(recs[2 * (int64_t)q + 1].w)); }
 };
 
 // A staged row: its 126 column-occupancy bits and its 126 second-entry bits as
@@ -689,7 +706,8 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
     for (int i = threadIdx.x; i <= nrows; i += kSlabThreads) {
       int st = rs[row_lo + i] - pos_lo;
       if (i < nrows) {
-        uint4 m = gm[i], p = gr[i];
+        uint4 m = gm[i], p = make_uint4(0u, 0u, 0u, 0u);
+        if (m.w >> 31) p = gr[i];
         if (m.w >> 31) st |= kRowRepeat;  // bit 127 of the row's masks: a column repeats / holds a third entry
         if (p.w >> 31) st |= kRowTriple;
         m.w &= 0x3fffffffu;
@@ -703,20 +721,21 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
       s_rs[i] = st;
     }
     for (int i = threadIdx.x; i < pos_hi - pos_lo; i += kSlabThreads) {
-      s_cand[i] = b.cand[pos_lo + i];
-      s_col[i] = (uint8_t)b.scol[pos_lo + i];
+      s_cand[i] = b.rec[2 * (int64_t)(pos_lo + i)];
+      s_col[i] = (uint8_t)bins_col(__float_as_int(b.rec[2 * (int64_t)(pos_lo + i) + 1].w));
     }
     __syncthreads();
   }
   RowsStaged sv{s_mask, s_rep, s_rs, s_before, s_cand, s_col, row_lo};
-  RowsGlobal gv{b.row_mask + 2 * rbase, rs, b.cand, b.scol};
+  RowsGlobal gv{b.row_mask + 2 * rbase, rs, b.rec};
   const int64_t es = b.offsets[e];
   const int tid = threadIdx.x;
   // the query rows hold only accepted clusters (rejected ones are in the
   // event's last row); a query's own data is read in sorted order
-  auto query = [&](int p, bool* inside) {
-    const float4 qr = b.qrec[p];
-    const float4 cr = staged ? s_cand[p - pos_lo] : b.cand[p];
+  auto query = [&](int p, bool* inside, int* idx) {
+    const float4 qr = b.rec[2 * (int64_t)p + 1];
+    const float4 cr = staged ? s_cand[p - pos_lo] : b.rec[2 * (int64_t)p];
+    *idx = __float_as_int(qr.y);
     const int bins = __float_as_int(qr.w);
     Query3 Q;
     Q.li = bins & 0x7ff;
@@ -726,7 +745,7 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
     Q.energy = cr.z;
     Q.phi = cr.y;
     Q.z = qr.x;
-    Q.r0 = qr.y;
+    Q.r0 = __fmul_rn(cr.x, qr.x);
     Q.aux = kDensity ? qr.z : cr.w;
     int lo, hi;
     layer_window(Q.li, sib, P.n_layers, kDensity ? 0 : 1, &lo, &hi);
@@ -736,8 +755,9 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
   };
   for (int p = q_lo + tid; p < q_hi; p += kSlabThreads) {
     bool inside;
-    const Query3 Q = query(p, &inside);
-    const int64_t gi = es + b.sorted[p];
+    int idx;
+    const Query3 Q = query(p, &inside, &idx);
+    const int64_t gi = es + idx;
     // staged windows: the rows holding an entry first, in one uniform pass
     unsigned long long live = 0;
     bool by_live = false;
@@ -751,7 +771,7 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
       else if (inside) search_all<true>(sv, P, Q, rho);
       else search_all<true>(gv, P, Q, rho);
       b.rho[gi] = rho;
-      reinterpret_cast<float*>(b.cand)[4 * (int64_t)p + 3] = rho;
+      reinterpret_cast<float*>(b.rec)[8 * (int64_t)p + 3] = rho;
     } else {
       Nh3 o;
       if (by_live) search_live<false>(sv, P, Q, live, o);
@@ -761,7 +781,7 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
       const bool found = o.best != FLT_MAX;
       const float dt = found ? o.best_t : FLT_MAX;
       const int dl = found ? o.best_l : INT_MAX, nl = found ? o.nl : -1;
-      const int ni = found ? b.sorted[o.nq] : -1;
+      const int ni = found ? __float_as_int(b.rec[2 * (int64_t)o.nq + 1].y) : -1;
       b.delta_t[gi] = dt;
       b.delta_l[gi] = dl;
       b.nh_l[gi] = nl;
@@ -780,37 +800,33 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
 }
 
 
-// One block per event: trackster ids by seed rank in index order, then each
-// cluster's walk along nearestHigher to its root and its label (replaces the
-// LIFO propagation).  par holds event-local indices.  Eight clusters per
-// thread and scan round, and one walk instead of rounds of pointer jumping
-// over the event: 20 -> XX us on one event of 5,000 clusters (a launch of one
-// block), 0.153 -> XX ms on 1,000 events.
-constexpr int kFinishThreads = 512;
-constexpr int kFinishPer = 8;
+// One block per event: trackster ids by seed rank in index order, eight
+// clusters per thread and scan round; clusters without a place in the rows
+// become roots of their own.
+constexpr int kRankThreads = 512;
+constexpr int kRankPer = 8;
 
-__global__ void __launch_bounds__(kFinishThreads) k3_finish(Batch3D b) {
-  pdl_wait();
+__global__ void __launch_bounds__(kRankThreads) k3_rank(Batch3D b) {
+  pdl_begin();
   const int e = blockIdx.x;
   const int64_t es = b.offsets[e];
   const int n = (int)(b.offsets[e + 1] - es);
-  int32_t* par = b.par + es;
   int32_t* ti = b.ti + es;
   int32_t* seed = b.seed + es;
-  __shared__ int s_w[kFinishThreads / 32];
+  __shared__ int s_w[kRankThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base_rank = 0;
-  for (int base = 0; base < n; base += kFinishThreads * kFinishPer) {
-    const int i0 = base + threadIdx.x * kFinishPer;
-    int f[kFinishPer], sum = 0;
+  for (int base = 0; base < n; base += kRankThreads * kRankPer) {
+    const int i0 = base + threadIdx.x * kRankPer;
+    int f[kRankPer], sum = 0;
 #pragma unroll
-    for (int j = 0; j < kFinishPer; ++j) f[j] = i0 + j < n ? seed[i0 + j] : 0;
+    for (int j = 0; j < kRankPer; ++j) f[j] = i0 + j < n ? seed[i0 + j] : 0;
 #pragma unroll
-    for (int j = 0; j < kFinishPer; ++j) {
-      if (f[j] < 0) {  // rejected by k3_key: no seed, a root of its own
+    for (int j = 0; j < kRankPer; ++j) {
+      if (f[j] < 0) {
         f[j] = 0;
         seed[i0 + j] = 0;
-        par[i0 + j] = -3;
+        b.par[es + i0 + j] = -3;
       }
       sum += f[j];
     }
@@ -824,13 +840,13 @@ __global__ void __launch_bounds__(kFinishThreads) k3_finish(Batch3D b) {
     __syncthreads();
     int before = 0, total = 0;
 #pragma unroll
-    for (int w = 0; w < kFinishThreads / 32; ++w) {
+    for (int w = 0; w < kRankThreads / 32; ++w) {
       if (w < warp) before += s_w[w];
       total += s_w[w];
     }
     int rank = base_rank + before + x - sum;
 #pragma unroll
-    for (int j = 0; j < kFinishPer; ++j)
+    for (int j = 0; j < kRankPer; ++j)
       if (f[j]) ti[i0 + j] = rank++;
     base_rank += total;
     __syncthreads();
@@ -839,34 +855,47 @@ __global__ void __launch_bounds__(kFinishThreads) k3_finish(Batch3D b) {
     b.ev_seeds[e] = base_rank;
     if (b.host_nt) b.host_nt[e] = base_rank;
   }
-  if (e == 0 && threadIdx.x < kFlagCount && b.host_flags) b.host_flags[threadIdx.x] = b.flags[threadIdx.x];
-  // walks of 64 steps without a root leave their pointer at the farthest
-  // cluster reached and are taken up again in another pass
-  for (;;) {
-    int unresolved = 0;
-    for (int i = threadIdx.x; i < n; i += kFinishThreads) {
-      int r = i, p = par[i];
-      if (p == -2) continue;  // a seed: labelled above
-      for (int step = 0; p >= 0 && step < 64; ++step) {
-        r = p;
-        p = par[r];
-      }
-      if (p < 0) {
-        ti[i] = p == -2 ? ti[r] : -1;
-      } else {
-        par[i] = r;
-        unresolved = 1;
-      }
+}
+
+// Each cluster's walk along nearestHigher to its root, and its label (replaces
+// the LIFO propagation); par holds event-local indices.  Every 64 steps a walk
+// leaves its own pointer at the farthest cluster reached, so that walks that
+// come through it later skip those steps (every ancestor is a valid parent).
+// The walks of a batch run side by side in as many blocks as it has clusters
+// for: rounds of pointer jumping by one block per event took 20 us on one
+// event of 5,000 clusters and 0.153 ms on 1,000 events; ranks and walks as two
+// kernels 8 + 9 us and 0.055 + 0.085 ms.
+__global__ void k3_label(Batch3D b) {
+  pdl_wait();
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < kFlagCount && b.host_flags) b.host_flags[i] = b.flags[i];
+  if (i >= b.n_points) return;
+  int t;
+  int p = b.par[i];
+  if (p == -2) {
+    t = b.ti[i];  // a seed
+  } else {
+    int32_t* par = b.par + b.offsets[event_of_blk(b, i)];
+    int32_t* ti = b.ti + (par - b.par);
+    int r = -1;
+    for (int step = 1; p >= 0; ++step) {
+      r = p;
+      if ((step & 63) == 0) b.par[i] = r;
+      p = par[r];
     }
-    if (!__syncthreads_or(unresolved)) break;
+    t = p == -2 ? ti[r] : -1;
+    b.ti[i] = t;
   }
   if (b.host_out) {  // a small host run's outputs, array after array
-    const float* o[7] = {b.rho, b.delta_t, reinterpret_cast<const float*>(b.delta_l),
-                         reinterpret_cast<const float*>(b.nh_l), reinterpret_cast<const float*>(b.nh_i),
-                         reinterpret_cast<const float*>(b.seed), reinterpret_cast<const float*>(b.ti)};
-#pragma unroll
-    for (int k = 0; k < 7; ++k)
-      for (int i = threadIdx.x; i < n; i += kFinishThreads) b.host_out[k * b.n_points + es + i] = o[k][es + i];
+    float* o = b.host_out + i;
+    const int64_t N = b.n_points;
+    o[0] = b.rho[i];
+    o[N] = b.delta_t[i];
+    o[2 * N] = __int_as_float(b.delta_l[i]);
+    o[3 * N] = __int_as_float(b.nh_l[i]);
+    o[4 * N] = __int_as_float(b.nh_i[i]);
+    o[5 * N] = __int_as_float(b.seed[i]);
+    o[6 * N] = __int_as_float(t);
   }
 }
 
@@ -922,7 +951,8 @@ cudaError_t launch_clue3d(const Batch3D& b, const Params3D& p, cudaStream_t s) {
   }
   {
     NvtxRange r("clue3d/finish");
-    if ((err = launch_pdl(k3_finish, b.n_events, kFinishThreads, 0, s, b)) != cudaSuccess) return err;
+    if ((err = launch_pdl(k3_rank, b.n_events, kRankThreads, 0, s, b)) != cudaSuccess) return err;
+    if ((err = launch_pdl(k3_label, grid, T, 0, s, b)) != cudaSuccess) return err;
   }
   return cudaSuccess;
 }

@@ -46,8 +46,7 @@ Params3D make_params3d(const clue3d_params& q) {
 
 enum Slot3D : int {
   T_TABLES,  // event offsets | event of each 256-cluster block, as in the pinned staging
-  T_KEY, T_RCNT, T_RSTART, T_ARR, T_SORTED, T_SCOL, T_TMP, T_PAR, T_EVSEEDS, T_FLAGS, T_MASK, T_REP, T_CAND, T_QREC,
-  T_TCAND, T_TQREC,
+  T_KEY, T_RCNT, T_RSTART, T_ARR, T_PAR, T_EVSEEDS, T_FLAGS, T_MASK, T_REP, T_REC, T_TREC,
   T_IN,   // host runs: the 8 inputs, each N long, back to back
   T_OUT,  // host runs: the 7 outputs, likewise
   T_COUNT
@@ -115,13 +114,13 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     const int64_t n_blk = (N + 255) / 256;
     const size_t table_bytes = 8 * (size_t)(E + 1) + 4 * (size_t)n_blk;
     need[T_TABLES] = table_bytes;
-    need[T_KEY] = need[T_ARR] = need[T_SORTED] = need[T_SCOL] = need[T_TMP] = need[T_PAR] = 4 * (size_t)N;
+    need[T_KEY] = need[T_ARR] = need[T_PAR] = 4 * (size_t)N;
     need[T_RCNT] = 4 * (size_t)(E * n_rows);
     need[T_RSTART] = 4 * (size_t)(E * n_rows + 1);
     need[T_EVSEEDS] = 4 * (size_t)E;
     need[T_FLAGS] = 4 * kFlagCount;
     need[T_MASK] = need[T_REP] = 16 * (size_t)(E * n_rows);
-    need[T_CAND] = need[T_QREC] = need[T_TCAND] = need[T_TQREC] = 16 * (size_t)N;
+    need[T_REC] = need[T_TREC] = 32 * (size_t)N;
     if (host_io) {
       need[T_IN] = 32 * (size_t)N;
       need[T_OUT] = 28 * (size_t)N;
@@ -199,18 +198,13 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     b.row_cnt = static_cast<int32_t*>(P(T_RCNT));
     b.row_start = static_cast<int32_t*>(P(T_RSTART));
     b.arr = static_cast<int32_t*>(P(T_ARR));
-    b.sorted = static_cast<int32_t*>(P(T_SORTED));
-    b.scol = static_cast<int32_t*>(P(T_SCOL));
-    b.tmp = static_cast<int32_t*>(P(T_TMP));
     b.par = static_cast<int32_t*>(P(T_PAR));
     b.ev_seeds = static_cast<int32_t*>(P(T_EVSEEDS));
     b.flags = static_cast<int32_t*>(P(T_FLAGS));
     b.row_mask = static_cast<unsigned long long*>(P(T_MASK));
     b.row_rep = static_cast<unsigned long long*>(P(T_REP));
-    b.cand = static_cast<float4*>(P(T_CAND));
-    b.qrec = static_cast<float4*>(P(T_QREC));
-    b.tcand = static_cast<float4*>(P(T_TCAND));
-    b.tqrec = static_cast<float4*>(P(T_TQREC));
+    b.rec = static_cast<float4*>(P(T_REC));
+    b.trec = static_cast<float4*>(P(T_TREC));
     e = launch_clue3d(b, make_params3d(*prm), s);
     if (e != cudaSuccess) return cuda_error(e, "launching CLUE3D kernels");
     if (host_io && !staged) {

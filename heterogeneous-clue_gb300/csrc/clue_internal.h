@@ -196,13 +196,8 @@ struct Batch3D {
   int32_t* row_cnt = nullptr;  // [E * n_rows + 1]
   int32_t* row_start = nullptr;// [E * n_rows + 1]
   int32_t* arr = nullptr;      // [N] arrival slot of each cluster in its row
-  int32_t* sorted = nullptr;   // [N] event-local index, by (row, phi bin, index)
-  int32_t* scol = nullptr;     // [N] phi bin of sorted entries
-  float4* cand = nullptr;      // [N] by sorted position: {roa, phi, energy, rho} of the entry
-  float4* qrec = nullptr;      // [N] by sorted position: {z, roa * z, density threshold, layer | etaBin << 11 | phiBin << 17}
-  float4* tcand = nullptr;     // [N] cand records by scatter position
-  float4* tqrec = nullptr;     // [N] qrec records by scatter position
-  int32_t* tmp = nullptr;      // [N]
+  float4* rec = nullptr;       // [2 N] by sorted position (row, phi bin, index): the cluster's 32-byte record
+  float4* trec = nullptr;      // [2 N] the records by scatter position
   int32_t* par = nullptr;      // [N]
   int32_t* ev_seeds = nullptr; // [E] tracksters per event
   unsigned long long* row_mask = nullptr;  // [E * n_rows * 2] phi columns present in each row; bit 127: a column repeats
