@@ -306,31 +306,34 @@ struct RowsGlobal {
   __device__ __forceinline__ int col(int q) const { return bins_col(__float_as_int(recs[2 * (int64_t)q + 1].w)); }
 };
 
-// A staged row: its 126 column-occupancy bits and its 126 second-entry bits as
-// four 32-bit words each; its start, relative to the first staged entry, with
-// two flags on top; and its entries in the columns before each word, a byte
-// per word (at most two entries per column there).
+// A staged row: its 126 column-occupancy bits as four 32-bit words; its entries
+// in the columns before each word, a byte per word (at most two entries per
+// column there); and its start, relative to the first staged entry, with a slot
+// of second-entry words where a column holds two (few rows do) and two flags.
+// Rows with a third entry in a column, or beyond the slots, are walked, with
+// the columns read from the records in global memory.
+constexpr int kRowStartBits = 12, kRowSlotBits = 8;
 constexpr int kRowRepeat = 1 << 30;  // a column holds two entries
-constexpr int kRowTriple = 1 << 29;  // a column holds three or more
+constexpr int kRowWalk = 1 << 29;    // counted entry by entry
 struct RowsStaged {
   const uint32_t* mask;    // 4 words per staged row
-  const uint32_t* rep;     // 4 words per staged row
+  const uint32_t* rep;     // 4 words per slot
   const int32_t* rstart;
   const uint32_t* before;
   const float4* cand;
-  const uint8_t* scol;
-  int row_lo;  // first staged row
-  __device__ __forceinline__ unsigned long long m0(int r) const { return word64(mask, r, 0); }
+  const float4* recs;      // the first staged entry's record in global memory
+  int row_lo;              // first staged row
+  __device__ __forceinline__ unsigned long long m0(int r) const { return word64(r, 0); }
   __device__ __forceinline__ unsigned long long m1(int r) const {
-    return word64(mask, r, 2) | ((rstart[r - row_lo] & kRowRepeat) ? 1ull << 63 : 0ull);
+    return word64(r, 2) | ((rstart[r - row_lo] & kRowRepeat) ? 1ull << 63 : 0ull);
   }
-  __device__ __forceinline__ unsigned long long word64(const uint32_t* m, int r, int w) const {
-    const uint32_t* p = m + 4 * (r - row_lo) + w;
+  __device__ __forceinline__ unsigned long long word64(int r, int w) const {
+    const uint32_t* p = mask + 4 * (r - row_lo) + w;
     return ((unsigned long long)p[1] << 32) | p[0];
   }
-  __device__ __forceinline__ int start(int r) const { return rstart[r - row_lo] & (kRowTriple - 1); }
+  __device__ __forceinline__ int start(int r) const { return rstart[r - row_lo] & ((1 << kRowStartBits) - 1); }
   __device__ __forceinline__ float4 rec(int q) const { return cand[q]; }
-  __device__ __forceinline__ int col(int q) const { return scol[q]; }
+  __device__ __forceinline__ int col(int q) const { return bins_col(__float_as_int(recs[2 * (int64_t)q + 1].w)); }
 };
 
 // Visits the entries of rows [s, t) whose phi column lies in the window
@@ -558,12 +561,12 @@ __device__ __forceinline__ RowRuns row_runs(const RowsStaged& v, int r, const Ph
   const int rs = v.rstart[i];
   const unsigned below = (1u << f.sh) - 1u;
   RowRuns o;
-  o.s = rs & (kRowTriple - 1);
+  o.s = rs & ((1 << kRowStartBits) - 1);
   o.na = __popc(f.arc_a(w));
   o.nb = f.wraps() ? __popc(f.arc_b(w)) : 0;
   o.qa = o.s + (int)((v.before[i] >> (8 * f.word)) & 0xffu) + __popc(w[f.word] & below);
-  if (rs & (kRowRepeat | kRowTriple)) {
-    if (rs & kRowTriple) {
+  if (rs & kRowRepeat) {
+    if (rs & kRowWalk) {
       const int t = v.start(r + 1);
       const int a0 = 32 * f.word + f.sh, n = f.all == 31u ? 5 : (f.all == 7u ? 3 : 1);
       int before = 0;
@@ -576,7 +579,7 @@ __device__ __forceinline__ RowRuns row_runs(const RowsStaged& v, int r, const Ph
       }
       o.qa = o.s + before;
     } else {
-      const uint32_t* p = v.rep + 4 * i;
+      const uint32_t* p = v.rep + 4 * ((rs >> kRowStartBits) & ((1 << kRowSlotBits) - 1));
       o.na += __popc(f.arc_a(p));
       o.nb += f.wraps() ? __popc(f.arc_b(p)) : 0;
       o.qa += __popc(p[f.word] & below);
@@ -658,9 +661,11 @@ __device__ __forceinline__ void search_live(const RowsStaged& v, const Params3D&
 
 // Staging of the searches: one block per (event, slab of kSlabLayers
 // layers).  The block copies the rows of the slab's layers and of the
-// sibling layers around them (occupancy masks, row starts, phi columns and
-// the 16-byte candidate records) into shared memory once, then runs the
-// searches of the slab's clusters from there (4 blocks of 256 threads per SM;
+// sibling layers around them (occupancy words, row starts and the 16-byte
+// candidate halves of the records) into shared memory once, then runs the
+// searches of the slab's clusters from there (5 blocks of 256 threads per SM,
+// since the searches wait on latency: 4 blocks, with second-entry words for every
+// row and the columns staged as well, 0.86 + 0.64 ms against 0.80 + 0.60;
 // slabs of 2, 6 and 8 layers measured slower or the same).  A cluster whose window leaves
 // the staged rows (the phi bin 126 quirk can move a cluster into the next
 // layer's first row) and a slab larger than the staging area read the global
@@ -670,19 +675,22 @@ constexpr int kSlabLayers = 4;
 constexpr int kSlabThreads = 256;
 constexpr int kSlabMaxRows = 384;  // 10 layers of rows and one more: sibling windows up to +-3 layers
 constexpr int kSlabMaxCand = 2048;
-// candidate records, row words, row starts and counts, phi columns
-constexpr size_t kSlabSmem = 16 * (size_t)kSlabMaxCand + 32 * (size_t)kSlabMaxRows + 8 * (size_t)(kSlabMaxRows + 1) +
-                             (size_t)kSlabMaxCand;
+constexpr int kSlabSlots = 128;
+static_assert(kSlabMaxCand < 1 << kRowStartBits && kSlabSlots <= 1 << kRowSlotBits, "packed row starts");
+// candidate records, row words, second-entry words, row starts and counts
+constexpr size_t kSlabSmem = 16 * (size_t)kSlabMaxCand + 16 * (size_t)kSlabMaxRows + 16 * (size_t)kSlabSlots +
+                             8 * (size_t)(kSlabMaxRows + 1);
 
 template <bool kDensity>
-__global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D P, int n_slabs) {
+__global__ void __launch_bounds__(kSlabThreads, 5) k3_search(Batch3D b, Params3D P, int n_slabs) {
   extern __shared__ __align__(16) unsigned char sm3[];
   float4* s_cand = reinterpret_cast<float4*>(sm3);
   uint32_t* s_mask = reinterpret_cast<uint32_t*>(s_cand + kSlabMaxCand);
   uint32_t* s_rep = s_mask + 4 * kSlabMaxRows;
-  int32_t* s_rs = reinterpret_cast<int32_t*>(s_rep + 4 * kSlabMaxRows);
+  int32_t* s_rs = reinterpret_cast<int32_t*>(s_rep + 4 * kSlabSlots);
   uint32_t* s_before = reinterpret_cast<uint32_t*>(s_rs + kSlabMaxRows + 1);
-  uint8_t* s_col = reinterpret_cast<uint8_t*>(s_before + kSlabMaxRows + 1);
+  __shared__ int s_slots;
+  if (threadIdx.x == 0) s_slots = 0;
   pdl_begin();
   const int e = blockIdx.x / n_slabs;
   const int L0 = (blockIdx.x % n_slabs) * kSlabLayers;
@@ -701,19 +709,22 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
   const int pos_lo = rs[row_lo], pos_hi = rs[row_hi + 1];
   const bool staged = nrows <= kSlabMaxRows && pos_hi - pos_lo <= kSlabMaxCand;
   if (staged) {
+    __syncthreads();  // s_slots
     const uint4* gm = reinterpret_cast<const uint4*>(b.row_mask + 2 * (rbase + row_lo));
     const uint4* gr = reinterpret_cast<const uint4*>(b.row_rep + 2 * (rbase + row_lo));
     for (int i = threadIdx.x; i <= nrows; i += kSlabThreads) {
       int st = rs[row_lo + i] - pos_lo;
       if (i < nrows) {
         uint4 m = gm[i], p = make_uint4(0u, 0u, 0u, 0u);
-        if (m.w >> 31) p = gr[i];
-        if (m.w >> 31) st |= kRowRepeat;  // bit 127 of the row's masks: a column repeats / holds a third entry
-        if (p.w >> 31) st |= kRowTriple;
+        if (m.w >> 31) {  // bit 127 of the row's masks: a column repeats / holds a third entry
+          p = gr[i];
+          const int slot = atomicAdd(&s_slots, 1);
+          st |= kRowRepeat | (slot < kSlabSlots ? slot << kRowStartBits : kRowWalk) | (p.w >> 31 ? kRowWalk : 0);
+          p.w &= 0x3fffffffu;
+          if (slot < kSlabSlots) reinterpret_cast<uint4*>(s_rep)[slot] = p;
+        }
         m.w &= 0x3fffffffu;
-        p.w &= 0x3fffffffu;
         reinterpret_cast<uint4*>(s_mask)[i] = m;
-        reinterpret_cast<uint4*>(s_rep)[i] = p;
         const unsigned c0 = __popc(m.x) + __popc(p.x), c1 = c0 + __popc(m.y) + __popc(p.y),
                        c2 = c1 + __popc(m.z) + __popc(p.z);
         s_before[i] = (c0 << 8) | (c1 << 16) | (c2 << 24);
@@ -722,11 +733,10 @@ __global__ void __launch_bounds__(kSlabThreads, 4) k3_search(Batch3D b, Params3D
     }
     for (int i = threadIdx.x; i < pos_hi - pos_lo; i += kSlabThreads) {
       s_cand[i] = b.rec[2 * (int64_t)(pos_lo + i)];
-      s_col[i] = (uint8_t)bins_col(__float_as_int(b.rec[2 * (int64_t)(pos_lo + i) + 1].w));
     }
     __syncthreads();
   }
-  RowsStaged sv{s_mask, s_rep, s_rs, s_before, s_cand, s_col, row_lo};
+  RowsStaged sv{s_mask, s_rep, s_rs, s_before, s_cand, b.rec + 2 * (int64_t)pos_lo, row_lo};
   RowsGlobal gv{b.row_mask + 2 * rbase, rs, b.rec};
   const int64_t es = b.offsets[e];
   const int tid = threadIdx.x;

@@ -1,0 +1,48 @@
+"""CLUE3D rows at the limits of the staged searches: columns held twice in more
+rows of a slab than it has second-entry slots, columns held three times and
+more (rows walked entry by entry), and phi on the edges of the 32-column words
+and of the wrap.  Bit-exact against the oracle."""
+import math
+
+import numpy as np
+import pytest
+
+import clue_gb300 as C
+import oracle
+from clue_gb300 import synthetic as S
+
+from _util import assert_bitexact
+
+pytestmark = pytest.mark.gpu
+
+NAMES = dict(rho="rho", delta_transverse="delta_t", delta_layers="delta_l", nh_layer="nh_layer", nh_index="nh_idx",
+             isSeed="isSeed", tracksterIndex="tracksterIndex")
+
+
+def _event(kind):
+    ev = S.clue3d_event(5, n_clusters=6000, n_layers=94)
+    rng = np.random.default_rng(9)
+    if kind == "pairs":  # every second cluster beside the one before it: nearly every row repeats a column
+        for k in ("eta", "phi", "layer", "z", "r_over_absz"):
+            ev[k][1::2] = ev[k][0::2]
+    elif kind == "triples":  # a narrow phi band: three entries and more in most columns
+        ev["phi"] = rng.uniform(-0.3, 0.3, ev["phi"].size).astype(np.float32)
+    else:  # a few ulps around every bin edge that starts a word, and around the wrap
+        edges = np.array([32, 64, 96, 124, 125, 126, 0, 1, 2], np.float64) * (2 * math.pi / 126) - math.pi
+        phi = rng.choice(edges, ev["phi"].size).astype(np.float32)
+        phi = (phi + rng.integers(-3, 4, phi.size).astype(np.float32) * np.float32(2.4e-7)).astype(np.float32)
+        ev["phi"] = np.clip(phi, -np.float32(math.pi), np.float32(math.pi))
+    return ev
+
+
+@pytest.mark.parametrize("siblings", [2, 3])
+@pytest.mark.parametrize("kind", ["pairs", "triples", "edges"])
+def test_rows(cuda_lib, kind, siblings):
+    ev = _event(kind)
+    prm = dict(n_layers=94, density_sibling_layers=siblings, nh_sibling_layers=siblings)
+    algo = C.Clusterizer(1.3, 2.0, 2.0)
+    out, nts = algo.run_clue3d(np.array([0, ev["z"].size], np.int64), ev, params=prm)
+    algo.close()
+    want, nt = oracle.clue3d(ev, **prm)
+    assert int(nts[0]) == nt
+    assert_bitexact({NAMES[k]: v for k, v in out.items()}, want, keys=tuple(NAMES.values()), label=kind)
