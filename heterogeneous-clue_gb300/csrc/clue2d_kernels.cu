@@ -954,6 +954,9 @@ __global__ void __launch_bounds__(kChunkThreads) k_seed_rank(Batch2D b) {
   }
 }
 
+// kHostOut: a small host run, whose outputs also go to the page-locked staging
+// (an instantiation of its own: the branch cost the others 0.1 ms per 65M points).
+template <bool kHostOut>
 __global__ void __launch_bounds__(kChunkThreads) k_label(Batch2D b) {
   const int c = blockIdx.x;
   __shared__ int s_e;
@@ -990,7 +993,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_label(Batch2D b) {
     const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
     if (i < i1 && v[j] <= -2) b.ci[i] = r[j];
   }
-  if (b.host_out) {  // a small host run's outputs, array after array
+  if constexpr (kHostOut) {
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
@@ -1049,7 +1052,8 @@ cudaError_t prepare_clue2d_kernels(int device) {
   const void* rest[] = {reinterpret_cast<const void*>(k_init), reinterpret_cast<const void*>(k_count),
                         reinterpret_cast<const void*>(k_layer_scan), reinterpret_cast<const void*>(k_order),
                         reinterpret_cast<const void*>(k_scatter), reinterpret_cast<const void*>(k_seed_chunk_scan),
-                        reinterpret_cast<const void*>(k_seed_rank), reinterpret_cast<const void*>(k_label)};
+                        reinterpret_cast<const void*>(k_seed_rank), reinterpret_cast<const void*>(k_label<false>),
+                        reinterpret_cast<const void*>(k_label<true>)};
   for (const void* f : rest) {
     cudaFuncAttributes a;
     if ((e = cudaFuncGetAttributes(&a, f)) != cudaSuccess) return e;
@@ -1225,7 +1229,9 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
   mark(6);
   {
     NvtxRange r("clue2d/label");
-    if ((err = launch_pdl(k_label, nc, kChunkThreads, 0, s, b)) != cudaSuccess) return err;
+    err = b.host_out ? launch_pdl(k_label<true>, nc, kChunkThreads, 0, s, b)
+                     : launch_pdl(k_label<false>, nc, kChunkThreads, 0, s, b);
+    if (err != cudaSuccess) return err;
   }
   mark(7);
   if (kernels) *kernels += 8 + (b.use_order ? 1 : 0) + (two_class ? 1 : 0);
