@@ -746,8 +746,15 @@ __global__ void __launch_bounds__(kSizeBuckets) k_order(Batch2D b) {
   int total;
   const int inc = block_inclusive_scan<kSizeBuckets>(v, s_ws, &total);
   s_base[tid] = inc - v;
-  if (blockIdx.x == 0 && tid == 0) b.flags[kFlagOrdered] = total;
   __syncthreads();
+  if (blockIdx.x == 0 && tid == 0) {
+    // the large layers come first in the order: the large-layer pass takes
+    // those, the other pass's tickets start behind them
+    const int big = b.order_big > 0 ? s_base[b.order_big] : 0;
+    b.flags[kFlagOrdered] = total;
+    b.flags[kFlagBigCount] = big;
+    b.flags[kFlagTicket] = big;
+  }
   const int e = (blockIdx.x * blockDim.x + tid) >> 5;
   if (e >= b.n_events) return;
   const int lane = lane_id();
@@ -825,7 +832,9 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
 // handles layers of at most max_m points on chip with `cap` points of shared
 // memory (several CTAs per SM); larger layers are appended to a list that the
 // second pass (big_pass = 1, launched with a large `cap` and fewer CTAs per
-// SM) drains.  Layers above `cap` in either pass use HBM scratch.
+// SM) drains.  Layers above `cap` in either pass use HBM scratch.  In an
+// ordered batch both lists are known beforehand (the order's two ends), and the
+// passes run beside one another, see launch_clue2d.
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_layers(Batch2D b, Params2D P, int cap, int max_m, int big_pass) {
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -1009,21 +1018,29 @@ __global__ void __launch_bounds__(kChunkThreads) k_label(Batch2D b) {
   }
 }
 
+// Beside event dependencies a kernel is launched the ordinary way (its
+// pdl_wait() then has nothing to wait for).
+enum LaunchKind { kDependent, kOrdinary };
+
 template <int NT>
 cudaError_t launch_layers(const Batch2D& b, const Params2D& p, int cap, int max_m, int big_pass, int grid,
-                          cudaStream_t s) {
+                          cudaStream_t s, LaunchKind kind) {
   Tuning2D t;
   t.layer_capacity = cap;
+  if (kind == kOrdinary) {
+    k_layers<NT><<<grid, NT, layer_smem_bytes(t), s>>>(b, p, cap, max_m, big_pass);
+    return cudaGetLastError();
+  }
   return launch_pdl(k_layers<NT>, grid, NT, layer_smem_bytes(t), s, b, p, cap, max_m, big_pass);
 }
 
 cudaError_t launch_layers_any(int threads, const Batch2D& b, const Params2D& p, int cap, int max_m, int big_pass,
-                              int grid, cudaStream_t s) {
+                              int grid, cudaStream_t s, LaunchKind kind) {
   switch (threads) {
-    case 128: return launch_layers<128>(b, p, cap, max_m, big_pass, grid, s);
-    case 256: return launch_layers<256>(b, p, cap, max_m, big_pass, grid, s);
-    case 1024: return launch_layers<1024>(b, p, cap, max_m, big_pass, grid, s);
-    default: return launch_layers<512>(b, p, cap, max_m, big_pass, grid, s);
+    case 128: return launch_layers<128>(b, p, cap, max_m, big_pass, grid, s, kind);
+    case 256: return launch_layers<256>(b, p, cap, max_m, big_pass, grid, s, kind);
+    case 1024: return launch_layers<1024>(b, p, cap, max_m, big_pass, grid, s, kind);
+    default: return launch_layers<512>(b, p, cap, max_m, big_pass, grid, s, kind);
   }
 }
 
@@ -1137,19 +1154,41 @@ int layer_grid(const Tuning2D& t, int n_items) {
   return g < 1 ? 1 : g;
 }
 
+// Largest layers first only where a pass ends on a visible tail: a few
+// layers per CTA (a sub-batch, a served batch).  With one layer per CTA or
+// less (a single event) every layer starts at once, and with hundreds per
+// CTA the tail is negligible and the event order measured faster.
+bool layers_ordered(const Tuning2D& t, int n_items) {
+  const int g = layer_grid(t, n_items);
+  return n_items > g && n_items <= 64 * g;
+}
+
 cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2D& t, cudaStream_t s,
-                          cudaEvent_t* ev, int64_t* kernels) {
+                          cudaEvent_t* ev, int64_t* kernels, const SideStream* side) {
   if (batch.n_events <= 0 || batch.n_points <= 0) return cudaSuccess;
-  // Largest layers first only where a pass ends on a visible tail: a few
-  // layers per CTA (a sub-batch, a served batch).  With one layer per CTA or
-  // less (a single event) every layer starts at once, and with hundreds per
-  // CTA the tail is negligible and the event order measured faster.
   Batch2D b = batch;
+  const int n_items = b.n_events * kLayers;
+  // No more layers than SMs (a single event): one pass of the widest CTA per
+  // layer, so that each layer's phases spread over 32 warps and large layers
+  // stay on chip.  Measured per producer call: 0.177 -> 0.131 ms on events of
+  // 150k-200k points, 0.136 -> 0.117 ms on 50k-150k, 0.113 -> 0.101 ms on 5k-20k.
+  Tuning2D tt = t;
   {
-    const int n_items = b.n_events * kLayers;
-    const int g = layer_grid(t, n_items);
-    b.use_order = (n_items > g && n_items <= 64 * g) ? 1 : 0;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (n_items <= sms) {
+      tt.threads = 1024;
+      tt.layer_capacity = std::max(std::max(t.layer_capacity, t.big_capacity), 4096);
+      tt.ctas_per_sm = 0;
+      tt.big_threads = tt.big_capacity = 0;
+    }
   }
+  const bool two_class = tt.big_threads > 0 && tt.big_capacity > tt.layer_capacity;
+  b.use_order = layers_ordered(t, n_items) ? 1 : 0;
+  // the size classes that may hold a layer above the first capacity; all of
+  // their layers fit the second one, or its HBM scratch
+  b.order_big = two_class ? kSizeBuckets - std::min(tt.layer_capacity >> 4, kSizeBuckets - 1) : 0;
   cudaError_t err;
   auto mark = [&](int i) {
     if (ev) cudaEventRecord(ev[i], s);
@@ -1182,44 +1221,50 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
     if ((err = launch_pdl(k_scatter, nc, kChunkThreads, 0, s, b)) != cudaSuccess) return err;
   }
   mark(3);
-  const int n_items = b.n_events * kLayers;
-  // No more layers than SMs (a single event): one pass of the widest CTA per
-  // layer, so that each layer's phases spread over 32 warps and large layers
-  // stay on chip.  Measured per producer call: 0.177 -> 0.131 ms on events of
-  // 150k-200k points, 0.136 -> 0.117 ms on 50k-150k, 0.113 -> 0.101 ms on 5k-20k.
-  Tuning2D tt = t;
-  {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (n_items <= sms) {
-      tt.threads = 1024;
-      tt.layer_capacity = std::max(std::max(t.layer_capacity, t.big_capacity), 4096);
-      tt.ctas_per_sm = 0;
-      tt.big_threads = tt.big_capacity = 0;
-    }
-  }
-  const bool two_class = tt.big_threads > 0 && tt.big_capacity > tt.layer_capacity;
   // Invariant: every layer-kernel grid is at most n_items = n_events * kLayers
   // (layer_grid caps it there).  The per-CTA HBM tile tables of the spill
   // path are sized on it: one table per (event, layer) at most, e.g. 100 for
   // a single event, which the allocation-free entry point relies on.
   {
     NvtxRange r("clue2d/layers");
-    err = launch_layers_any(tt.threads, b, p, tt.layer_capacity, two_class ? tt.layer_capacity : INT_MAX, 0,
-                            layer_grid(tt, n_items), s);
-    if (err == cudaSuccess && two_class) {
-      Tuning2D big;
-      big.threads = tt.big_threads;
-      big.layer_capacity = tt.big_capacity;
-      err = launch_layers_any(tt.big_threads, b, p, tt.big_capacity, INT_MAX, 1, layer_grid(big, n_items), s);
+    const int grid = layer_grid(tt, n_items);
+    const int max_m = two_class ? tt.layer_capacity : INT_MAX;
+    Tuning2D big;
+    big.threads = tt.big_threads;
+    big.layer_capacity = tt.big_capacity;
+    if (two_class && b.use_order) {
+      // The large layers on this stream, the others from the same point on the
+      // side stream: the CTAs of the pass over the small layers start as those
+      // of the large pass run out of layers, instead of after the last one has
+      // ended, and the large layers start first, not last (48 uneven events 295
+      // -> 261 us; 200 HGCAL events, all of whose layers are large, 5.61 -> 5.58 ms).
+      Batch2D large = b;
+      large.cursor = b.order;  // the list that the large-layer pass drains
+      cudaStream_t s2 = side ? side->stream : s;
+      if (side && (err = cudaEventRecord(side->fork, s)) != cudaSuccess) return err;
+      err = launch_layers_any(big.threads, large, p, big.layer_capacity, INT_MAX, 1, layer_grid(big, n_items), s,
+                              kOrdinary);
+      if (err == cudaSuccess && side) err = cudaStreamWaitEvent(s2, side->fork, 0);
+      if (err == cudaSuccess) err = launch_layers_any(tt.threads, b, p, tt.layer_capacity, max_m, 0, grid, s2, kOrdinary);
+      if (err == cudaSuccess && side) err = cudaEventRecord(side->join, s2);
+      if (err == cudaSuccess && side) err = cudaStreamWaitEvent(s, side->join, 0);
+    } else {
+      err = launch_layers_any(tt.threads, b, p, tt.layer_capacity, max_m, 0, grid, s, kDependent);
+      if (err == cudaSuccess && two_class)
+        err = launch_layers_any(big.threads, b, p, big.layer_capacity, INT_MAX, 1, layer_grid(big, n_items), s, kDependent);
     }
   }
   if (err != cudaSuccess) return err;
   mark(4);
   {
     NvtxRange r("clue2d/seed_chunk_scan");
-    if ((err = launch_pdl(k_seed_chunk_scan, warps_grid, 256, 0, s, b)) != cudaSuccess) return err;
+    if (two_class && b.use_order) {  // behind the join of the two passes
+      k_seed_chunk_scan<<<warps_grid, 256, 0, s>>>(b);
+      err = cudaGetLastError();
+    } else {
+      err = launch_pdl(k_seed_chunk_scan, warps_grid, 256, 0, s, b);
+    }
+    if (err != cudaSuccess) return err;
   }
   mark(5);
   {

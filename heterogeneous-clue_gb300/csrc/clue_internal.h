@@ -43,7 +43,7 @@ enum FlagSlot : int {
   kFlagTicket = 2,
   kFlagSpilled = 3,
   kFlagTicket2 = 4,   // ticket of the large-layer pass
-  kFlagBigCount = 5,  // layers left to the large-layer pass
+  kFlagBigCount = 5,  // layers of the large-layer pass
   kFlagOrdered = 6,   // non-empty layers in the size order
   kFlagCount = 8
 };
@@ -106,6 +106,7 @@ struct Batch2D {
   int32_t* lstart = nullptr;  // [E*100] first grouped position of (event, layer)
   int32_t* cursor = nullptr;  // [E*100]
   int32_t use_order = 0;         // set per launch: take the layers in `order`
+  int32_t order_big = 0;         // set per launch: size classes of the large-layer pass (0: one class of layers)
   int32_t* order = nullptr;      // [E*100] non-empty (event, layer) items, largest first
   int32_t* size_hist = nullptr;  // [2*kSizeBuckets] layers per size class, then cursors
   float* gx = nullptr;        // [N] grouped copies, event-local index in gid
@@ -130,12 +131,23 @@ size_t layer_smem_bytes(const Tuning2D& t);
 // stream capture; again after the device's context was reset).
 cudaError_t prepare_clue2d_kernels(int device);
 
+// Whether a batch of n_items (event, layer) items takes its layers largest first.
+bool layers_ordered(const Tuning2D& t, int n_items);
+
+// A second stream and two events, for the pass over the small layers of an
+// ordered batch (without them it follows the pass over the large ones).
+struct SideStream {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+
 constexpr int kStages2D = 7;
 // Queues the whole 2D pipeline of one batch on `s`.  With `stage_events`
 // (kStages2D + 1 events) an event is recorded before each stage and after the
 // last; `kernels`, when given, is increased by the number of kernels queued.
 cudaError_t launch_clue2d(const Batch2D& b, const Params2D& p, const Tuning2D& t, cudaStream_t s,
-                          cudaEvent_t* stage_events = nullptr, int64_t* kernels = nullptr);
+                          cudaEvent_t* stage_events = nullptr, int64_t* kernels = nullptr,
+                          const SideStream* side = nullptr);
 
 // Adds an order-sensitive digest of n_words 32-bit words to *d_out.
 cudaError_t launch_digest(const void* words, int64_t n_words, unsigned long long* d_out, cudaStream_t s);

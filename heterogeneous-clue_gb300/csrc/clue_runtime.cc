@@ -214,6 +214,9 @@ Handle::~Handle() {
   if (done_event) cudaEventDestroy(done_event);
   for (auto ev : pipe_events)
     if (ev) cudaEventDestroy(ev);
+  for (auto ev : {side.fork, side.join})
+    if (ev) cudaEventDestroy(ev);
+  if (side.stream) cudaStreamDestroy(side.stream);
   if (copy_in) cudaStreamDestroy(copy_in);
   if (copy_out) cudaStreamDestroy(copy_out);
   arena.release();
@@ -226,6 +229,19 @@ int Handle::wait_previous() {
   pending = false;
   if (e != cudaSuccess) return cuda_error(e, "waiting for previous run");
   return CLUE_OK;
+}
+
+// The side stream of ordered batches, when this one may be one (outside any
+// stream capture of ours).
+int Handle::ensure_side(int n_events) {
+  if (side.join || !layers_ordered(tuning, n_events * kLayers)) return CLUE_OK;
+  cudaError_t e = side.stream ? cudaSuccess : cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking);
+  if (e != cudaSuccess) side.stream = nullptr;
+  for (auto* ev : {&side.fork, &side.join}) {
+    if (e != cudaSuccess || *ev) continue;
+    if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess) *ev = nullptr;
+  }
+  return e == cudaSuccess ? CLUE_OK : cuda_error(e, "side stream");
 }
 
 int Handle::check_device_flags() {
@@ -282,7 +298,7 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
       return cuda_error(e, "H2D points");
     }
   }
-  e = launch_clue2d(b, h->p2d, h->tuning, s, stage_events, kernels);
+  e = launch_clue2d(b, h->p2d, h->tuning, s, stage_events, kernels, h->side.join ? &h->side : nullptr);
   if (e != cudaSuccess) return cuda_error(e, "launching CLUE kernels");
   if (host_io && !b.host_out) {
     const clue_outputs* o = r.out;
@@ -409,6 +425,7 @@ int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nul
   rc = h->flags_host.reserve(4 * kFlagCount);
   if (rc) return rc;
 
+  if ((rc = h->ensure_side(r.E))) return rc;
   Batch2D b;
   fill_batch_views(h, r, nchunks, host_io, b, h->stage.p, static_cast<int32_t*>(h->flags_host.p));
 
@@ -710,7 +727,9 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
     if ((e = cudaStreamWaitEvent(cs, h2d[k], 0)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(cs, d2h[k], 0)) != cudaSuccess)
       return cuda_error(e, "sub-batch set-up");
-    if ((e = launch_clue2d(b, h->p2d, h->tuning, cs, nullptr, &kernels)) != cudaSuccess)
+    if ((rc = h->ensure_side(Es))) return rc;
+    if ((e = launch_clue2d(b, h->p2d, h->tuning, cs, nullptr, &kernels, h->side.join ? &h->side : nullptr)) !=
+        cudaSuccess)
       return cuda_error(e, "launching CLUE kernels");
     if ((e = cudaEventRecord(comp[k], cs)) != cudaSuccess) return cuda_error(e, "cudaEventRecord");
     const clue_outputs* o = r.out;

@@ -129,6 +129,7 @@ struct Handle {
   DeviceArena arena_pipe[kPipeSlots - 1];  // further slots of the pipelined host-memory path
   cudaStream_t copy_in = nullptr;         // pipelined host-memory path: H2D stream
   cudaStream_t copy_out = nullptr;        // and D2H stream
+  SideStream side;                        // small layers of ordered batches; created by the first of them
   cudaEvent_t pipe_events[3 * kPipeSlots] = {};  // per slot: H2D done, kernels done, D2H done
   clue_run_stats last_run{};              // copies and kernels of the last 2D run
   int64_t graph_kernels = 0;              // kernels in graph_exec
@@ -142,6 +143,7 @@ struct Handle {
 
   ~Handle();
   int wait_previous();
+  int ensure_side(int n_events);
   int check_device_flags();
   int profile_batch(int32_t E, const int64_t* off, const float* x, const float* y, const int32_t* layer,
                     const float* w, const clue_outputs* out, float* stage_ms);
