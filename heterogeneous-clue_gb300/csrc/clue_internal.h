@@ -33,6 +33,8 @@ constexpr int kTableStride = ((kTableInts * 4 + 15) / 16) * 4;
 // Points per event-aligned chunk of the streaming kernels (count, scatter, seed ranks).
 constexpr int kChunk = 4096;
 constexpr int kChunkThreads = 512;
+// 32-bit words of a chunk's seed bits.
+constexpr int kChunkWords = kChunk / 32;
 // Size classes of the largest-first layer order (16 points per class).
 constexpr int kSizeBuckets = 256;
 
@@ -115,7 +117,7 @@ struct Batch2D {
   int32_t* gid = nullptr;
   float* sp[8] = {};          // [N] each: HBM home of layers larger than layer_capacity
   int32_t* sp_tbl = nullptr;  // [grid * kTableInts]
-  int32_t* chunk_seeds = nullptr;  // [n_chunks]
+  uint32_t* seed_bits = nullptr;   // [n_chunks * kChunkWords] the seeds of each chunk
   int32_t* chunk_base = nullptr;   // [n_chunks]
   int32_t* flags = nullptr;        // [kFlagCount]
 };

@@ -53,8 +53,8 @@ constexpr size_t kOffLstart = kOffLcnt + al(4 * kLayers);                      /
 constexpr size_t kOffCursor = kOffLstart + al(4 * kLayers);                    // int32[100]
 constexpr size_t kOffOrder = kOffCursor + al(4 * kLayers);                     // int32[100 + 2 * size classes]
 constexpr size_t kOffFlags = kOffOrder + al(4 * (kLayers + 2 * kSizeBuckets));  // int32[kFlagCount]
-constexpr size_t kOffChunkSeeds = kOffFlags + al(4 * kFlagCount);              // int32[chunks]
-constexpr size_t kOffChunkBase = kOffChunkSeeds + al(4 * kNoAllocMaxChunks);   // int32[chunks]
+constexpr size_t kOffSeedBits = kOffFlags + al(4 * kFlagCount);                // uint32[chunks * words of a chunk]
+constexpr size_t kOffChunkBase = kOffSeedBits + al(4 * kChunkWords * kNoAllocMaxChunks);  // int32[chunks]
 constexpr size_t kOffGx = kOffChunkBase + al(4 * kNoAllocMaxChunks);           // 4 x [N] grouped copies
 constexpr size_t kOffSpRec = kOffGx + 4 * al(4 * kNoAllocMaxPoints);           // 16 B x N spill records
 constexpr size_t kOffSpNh = kOffSpRec + al(16 * kNoAllocMaxPoints);            // int32[N]
@@ -137,7 +137,7 @@ extern "C" int clue_run_event_noalloc(const clue_params* params, int32_t n, cons
   b.flags = reinterpret_cast<int32_t*>(base + kOffFlags);
   b.order = reinterpret_cast<int32_t*>(base + kOffOrder);
   b.size_hist = b.order + kLayers;
-  b.chunk_seeds = reinterpret_cast<int32_t*>(base + kOffChunkSeeds);
+  b.seed_bits = reinterpret_cast<uint32_t*>(base + kOffSeedBits);
   b.chunk_base = reinterpret_cast<int32_t*>(base + kOffChunkBase);
   const size_t plane = al(4 * kNoAllocMaxPoints);
   b.gx = reinterpret_cast<float*>(base + kOffGx);

@@ -155,7 +155,8 @@ std::vector<size_t> sizes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bo
   s[S_SP1] = s[S_SP2] = s[S_SP3] = s[S_SP6] = s[S_SP7] = 0;
   s[S_SP4] = s[S_SP5] = 4 * (size_t)N;
   s[S_SPTBL] = 4 * (size_t)kTableStride * grid;
-  s[S_CSEED] = s[S_CBASE] = 4 * (size_t)std::max<int64_t>(nchunks, 1);
+  s[S_CSEED] = 4 * kChunkWords * (size_t)std::max<int64_t>(nchunks, 1);
+  s[S_CBASE] = 4 * (size_t)std::max<int64_t>(nchunks, 1);
   s[S_FLAGS] = 4 * kFlagCount;
   s[S_ORDER] = 4 * ((size_t)E * kLayers + 2 * kSizeBuckets);
   if (host_io) {
@@ -374,7 +375,7 @@ void fill_batch_views(Handle* h, const Run2D& r, int64_t nchunks, bool host_io, 
   b.gid = static_cast<int32_t*>(P(S_GID));
   for (int i = 0; i < 8; ++i) b.sp[i] = static_cast<float*>(P(S_SP0 + i));
   b.sp_tbl = static_cast<int32_t*>(P(S_SPTBL));
-  b.chunk_seeds = static_cast<int32_t*>(P(S_CSEED));
+  b.seed_bits = static_cast<uint32_t*>(P(S_CSEED));
   b.chunk_base = static_cast<int32_t*>(P(S_CBASE));
   b.flags = static_cast<int32_t*>(P(S_FLAGS));
   b.order = static_cast<int32_t*>(P(S_ORDER));
