@@ -61,3 +61,47 @@ def test_fixed_point_forms(cuda_lib, kind, per_cluster):
             assert max_ulp(got[k], v) <= 1, k
         else:
             assert np.array_equal(got[k].view(np.int32), np.asarray(v).view(np.int32)), k
+
+
+@pytest.mark.parametrize("place", ["ring", "axes", "diagonal", "centre", "far"])
+def test_cluster_fields_over_their_ranges(cuda_lib, place):
+    """Positions and layer depths on both sides of every limit between the
+    two-float and the double forms: signs, the axes, equal coordinates, clusters
+    near the beam and far out, z negative, small against r, tiny and huge, and
+    clusters without weight."""
+    import torch
+    rng = np.random.default_rng(len(place))
+    n = 6000
+    phi = rng.uniform(-np.pi, np.pi, n)
+    r = {"ring": rng.uniform(20, 250, n), "axes": rng.uniform(0, 250, n), "diagonal": rng.uniform(1, 250, n),
+         "centre": 10.0 ** rng.uniform(-9, 0, n), "far": 10.0 ** rng.uniform(2, 4, n)}[place]
+    if place == "axes":
+        phi = np.round(phi / (np.pi / 2)) * (np.pi / 2)
+    if place == "diagonal":
+        phi = (np.round(phi / (np.pi / 2)) + 0.5) * (np.pi / 2)
+    x, y = (r * np.cos(phi)).astype(np.float32), (r * np.sin(phi)).astype(np.float32)
+    if place == "axes":
+        x[np.abs(x) < 1e-3] = 0
+        y[np.abs(y) < 1e-3] = 0
+    if place == "diagonal":
+        y = np.copysign(np.abs(x), y)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    w[rng.random(n) < 0.02] = 0
+    lz = np.concatenate([S.layer_z(), -S.layer_z(), np.array([1e-4, 0.01, 1, 20, 60, 250, 1e5, 1e7, -5], np.float32)])
+    lz = lz.astype(np.float32)
+    layer = rng.integers(0, lz.size, n).astype(np.int32)
+    ci = (np.arange(n) // 3).astype(np.int32)
+    seed = (np.arange(n) % 3 == 0).astype(np.int32)
+    off = np.array([0, n], np.int64)
+    _, want = OB.layer_clusters(off, x, y, layer, w, seed, ci, lz)
+    d = {k: torch.from_numpy(v).cuda() for k, v in dict(x=x, y=y, layer=layer, weight=w).items()}
+    o2 = dict(isSeed=torch.from_numpy(seed).cuda(), clusterIndex=torch.from_numpy(ci).cuda())
+    algo = C.Clusterizer(1.3, 2.0, 2.0)
+    _, got = algo.layer_clusters(off, d["x"], d["y"], d["layer"], d["weight"], o2, layer_z=lz)
+    got = {k: v.cpu().numpy() for k, v in got.items()}
+    algo.close()
+    for k, v in want.items():
+        if k in ("eta", "phi"):
+            assert max_ulp(got[k], v) <= 1, k
+        else:
+            assert np.array_equal(got[k].view(np.int32), np.asarray(v).view(np.int32)), k
