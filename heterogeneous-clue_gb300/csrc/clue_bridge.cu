@@ -30,7 +30,12 @@ namespace {
 constexpr double kWScale = 16777216.0;  // 2^24
 constexpr double kPScale = 65536.0;     // 2^16
 
-enum BridgeSlot { B_OFF, B_COFF, B_COUNT, B_ACC, B_SEED, B_LZ, B_FLAGS, B_CEV, B_SLOTS };
+enum BridgeSlot {
+  B_TABLES,  // event offsets | cluster offsets | layer z | event of each chunk, as in the pinned staging
+  B_COUNT,
+  B_SUMS,    // sums | seed of each cluster | status words: zero at the start of a build
+  B_SLOTS
+};
 
 // Points per block of the point kernels: each block finds the event of its
 // first point once and then follows event boundaries forwards.
@@ -407,11 +412,10 @@ int check_offsets(int32_t E, const int64_t* off, const char* what) {
 // Event of the first point of each chunk of kBridgeChunk points (empty
 // events own no point; the event of a point is the last e with off[e] <= i).
 void chunk_events(int32_t E, const int64_t* off, int nch, int32_t* cev) {
-  int32_t e = 0;
-  for (int c = 0; c < nch; ++c) {
-    const int64_t i = (int64_t)c * kBridgeChunk;
-    while (e + 1 < E && off[e + 1] <= i) ++e;
-    cev[c] = e;
+  int c = 0;
+  for (int32_t e = 0; e < E; ++e) {
+    const int end = e + 1 < E ? (int)std::min<int64_t>(chunks_for(off[e + 1]), nch) : nch;
+    for (; c < end; ++c) cev[c] = e;
   }
 }
 
@@ -448,28 +452,29 @@ int clue_bridge_count(clue_handle* hh, int32_t E, const int64_t* off, const int3
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
     if ((rc = h->wait_previous())) return rc;
     std::vector<size_t> need(clue::B_SLOTS, 0);
-    need[clue::B_OFF] = 8 * (size_t)(E + 1);
-    need[clue::B_COUNT] = 4 * (size_t)E;
     const int nch = clue::chunks_for(N);
-    need[clue::B_CEV] = 4 * (size_t)std::max(nch, 1);
+    const size_t table_bytes = 8 * (size_t)(E + 1) + 4 * (size_t)nch;
+    need[clue::B_TABLES] = table_bytes;
+    need[clue::B_COUNT] = 4 * (size_t)E;
     if ((rc = h->arena_bridge.reserve(need, clue::bridge_budget(h)))) return rc;
-    if ((rc = h->stage.reserve(8 * (size_t)(E + 1) + 4 * (size_t)nch))) return rc;
+    if ((rc = h->stage.reserve(table_bytes))) return rc;
+    if ((rc = h->nt_host.reserve(4 * (size_t)E))) return rc;
     auto P = [&](int s) { return h->arena_bridge.ptr(s); };
     cudaStream_t s = h->stream;
     memcpy(h->stage.p, off, 8 * (size_t)(E + 1));
     int32_t* cev = reinterpret_cast<int32_t*>(static_cast<char*>(h->stage.p) + 8 * (size_t)(E + 1));
     clue::chunk_events(E, off, nch, cev);
-    if ((e = cudaMemcpyAsync(P(clue::B_OFF), h->stage.p, 8 * (size_t)(E + 1), cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(P(clue::B_CEV), cev, 4 * (size_t)nch, cudaMemcpyHostToDevice, s)) ||
+    if ((e = cudaMemcpyAsync(P(clue::B_TABLES), h->stage.p, table_bytes, cudaMemcpyHostToDevice, s)) ||
         (e = cudaMemsetAsync(P(clue::B_COUNT), 0, 4 * (size_t)E, s)))
       return cuda_error(e, "bridge set-up");
+    const int64_t* d_off = static_cast<const int64_t*>(P(clue::B_TABLES));
     if (N > 0)
-      clue::k_bridge_count<<<nch, clue::kBridgeThreads, 0, s>>>(N, static_cast<const int64_t*>(P(clue::B_OFF)),
-                                                                  static_cast<const int32_t*>(P(clue::B_CEV)),
+      clue::k_bridge_count<<<nch, clue::kBridgeThreads, 0, s>>>(N, d_off,
+                                                                  reinterpret_cast<const int32_t*>(d_off + (E + 1)),
                                                                   isSeed, static_cast<int32_t*>(P(clue::B_COUNT)));
     if ((e = cudaGetLastError())) return cuda_error(e, "k_bridge_count");
-    std::vector<int32_t> counts(E);
-    if ((e = cudaMemcpyAsync(counts.data(), P(clue::B_COUNT), 4 * (size_t)E, cudaMemcpyDeviceToHost, s)) ||
+    const int32_t* counts = static_cast<const int32_t*>(h->nt_host.p);
+    if ((e = cudaMemcpyAsync(h->nt_host.p, P(clue::B_COUNT), 4 * (size_t)E, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
       return cuda_error(e, "bridge counts");
     for (int32_t i = 0; i < E; ++i) cluster_offsets[i + 1] = cluster_offsets[i] + counts[i];
@@ -500,17 +505,14 @@ int clue_bridge_build(clue_handle* hh, const clue_bridge_params* p, int32_t E, c
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
     if ((rc = h->wait_previous())) return rc;
     std::vector<size_t> need(clue::B_SLOTS, 0);
-    need[clue::B_OFF] = need[clue::B_COFF] = 8 * (size_t)(E + 1);
-    need[clue::B_COUNT] = 4 * (size_t)E;
-    need[clue::B_ACC] = 24 * (size_t)std::max<int64_t>(C, 1);
-    need[clue::B_SEED] = 4 * (size_t)std::max<int64_t>(C, 1);
-    need[clue::B_LZ] = 4 * (size_t)p->n_layers;
-    need[clue::B_FLAGS] = 4 * clue::kFlagCount;
     const int nch = clue::chunks_for(N);
-    need[clue::B_CEV] = 4 * (size_t)std::max(nch, 1);
+    const size_t table_bytes = 16 * (size_t)(E + 1) + 4 * (size_t)p->n_layers + 4 * (size_t)nch;
+    const size_t sum_bytes = 28 * (size_t)C + 4 * clue::kFlagCount;
+    need[clue::B_TABLES] = table_bytes;
+    need[clue::B_COUNT] = 4 * (size_t)E;
+    need[clue::B_SUMS] = sum_bytes;
     if ((rc = h->arena_bridge.reserve(need, clue::bridge_budget(h)))) return rc;
-    const size_t stage_bytes = 16 * (size_t)(E + 1) + 4 * (size_t)p->n_layers + 4 * (size_t)nch;
-    if ((rc = h->stage.reserve(stage_bytes))) return rc;
+    if ((rc = h->stage.reserve(table_bytes))) return rc;
     if ((rc = h->flags_host.reserve(4 * clue::kFlagCount))) return rc;
     auto P = [&](int s) { return h->arena_bridge.ptr(s); };
     char* st = static_cast<char*>(h->stage.p);
@@ -520,28 +522,23 @@ int clue_bridge_build(clue_handle* hh, const clue_bridge_params* p, int32_t E, c
     int32_t* cev = reinterpret_cast<int32_t*>(st + 16 * (size_t)(E + 1) + 4 * (size_t)p->n_layers);
     clue::chunk_events(E, off, nch, cev);
     cudaStream_t s = h->stream;
-    if ((e = cudaMemcpyAsync(P(clue::B_OFF), st, 8 * (size_t)(E + 1), cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(P(clue::B_COFF), st + 8 * (size_t)(E + 1), 8 * (size_t)(E + 1), cudaMemcpyHostToDevice,
-                             s)) ||
-        (e = cudaMemcpyAsync(P(clue::B_LZ), st + 16 * (size_t)(E + 1), 4 * (size_t)p->n_layers,
-                             cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemsetAsync(P(clue::B_ACC), 0, 24 * (size_t)std::max<int64_t>(C, 1), s)) ||
-        (e = cudaMemsetAsync(P(clue::B_SEED), 0, 4 * (size_t)std::max<int64_t>(C, 1), s)) ||
-        (e = cudaMemsetAsync(P(clue::B_FLAGS), 0, 4 * clue::kFlagCount, s)) ||
-        (e = cudaMemcpyAsync(P(clue::B_CEV), cev, 4 * (size_t)nch, cudaMemcpyHostToDevice, s)))
+    if ((e = cudaMemcpyAsync(P(clue::B_TABLES), st, table_bytes, cudaMemcpyHostToDevice, s)) ||
+        (e = cudaMemsetAsync(P(clue::B_SUMS), 0, sum_bytes, s)))
       return cuda_error(e, "bridge set-up");
-    int32_t* flags = static_cast<int32_t*>(P(clue::B_FLAGS));
-    auto* acc = static_cast<unsigned long long*>(P(clue::B_ACC));
-    auto* seed_of = static_cast<int32_t*>(P(clue::B_SEED));
+    const int64_t* d_off = static_cast<const int64_t*>(P(clue::B_TABLES));
+    const int64_t* d_coff = d_off + (E + 1);
+    const float* d_lz = reinterpret_cast<const float*>(d_coff + (E + 1));
+    const int32_t* d_cev = reinterpret_cast<const int32_t*>(d_lz + p->n_layers);
+    auto* acc = static_cast<unsigned long long*>(P(clue::B_SUMS));
+    auto* seed_of = reinterpret_cast<int32_t*>(acc + 3 * C);
+    int32_t* flags = seed_of + C;
     if (N > 0)
-      clue::k_bridge_accumulate<<<nch, clue::kBridgeThreads, 0, s>>>(
-          N, static_cast<const int64_t*>(P(clue::B_OFF)), static_cast<const int32_t*>(P(clue::B_CEV)),
-          static_cast<const int64_t*>(P(clue::B_COFF)), x, y, weight, isSeed, clusterIndex, acc, seed_of, flags);
+      clue::k_bridge_accumulate<<<nch, clue::kBridgeThreads, 0, s>>>(N, d_off, d_cev, d_coff, x, y, weight, isSeed,
+                                                                     clusterIndex, acc, seed_of, flags);
     if ((e = cudaGetLastError())) return cuda_error(e, "k_bridge_accumulate");
     if (C > 0)
       clue::k_bridge_finalize<<<clue::grid_for(C), 256, 0, s>>>(C, acc, seed_of, x, y, layer,
-                                                                 static_cast<const float*>(P(clue::B_LZ)),
-                                                                 p->n_layers, p->radius, p->isSilicon, *out, flags);
+                                                                 d_lz, p->n_layers, p->radius, p->isSilicon, *out, flags);
     if ((e = cudaGetLastError())) return cuda_error(e, "k_bridge_finalize");
     if ((e = cudaMemcpyAsync(h->flags_host.p, flags, 4 * clue::kFlagCount, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
