@@ -252,7 +252,9 @@ __device__ void order_queries(const LayerStore<TT, QT>& S, const int m, const fl
     const float2 p = rec_xy(S.rec[q]);
     const int bx0 = tile_bin(__fsub_rn(p.x, d)), bx1 = tile_bin(__fadd_rn(p.x, d));
     const int by0 = tile_bin(__fsub_rn(p.y, d)), by1 = tile_bin(__fadd_rn(p.y, d));
-    return NB - 1 - min(candidate_count(S.tbl, bx0, bx1, by0, by1) >> 1, NB - 1);  // 2 candidates per bucket
+    // 2 candidates per bucket; 8 for boxes of three columns and more, which would
+    // crowd the first bucket (the same event: 58.9 -> 57.2 us)
+    return NB - 1 - min(candidate_count(S.tbl, bx0, bx1, by0, by1) >> (d > 5.f ? 3 : 1), NB - 1);
   };
   for (int i = tid; i < NB; i += NT) s_bins[i] = 0;
   __syncthreads();
@@ -340,9 +342,15 @@ __device__ __forceinline__ void for_candidates(const TT* tbl, int bx0, int bx1, 
 #pragma unroll 4
     for (int t = 0; t < sg.total; ++t) visit(sg.at(t));
   } else {
+    // the next column's run is read while this one is walked (one toy event with
+    // dc 20 cm: 60.1 -> 58.9 us)
+    int k = (int)tbl[bx0 * kGridCols + by0], e = (int)tbl[bx0 * kGridCols + by1 + 1];
     for (int c = bx0; c <= bx1; ++c) {
-      const int e = (int)tbl[c * kGridCols + by1 + 1];
-      for (int k = (int)tbl[c * kGridCols + by0]; k < e; ++k) visit(k);
+      const int cn = min(c + 1, bx1) * kGridCols;
+      const int kn = (int)tbl[cn + by0], en = (int)tbl[cn + by1 + 1];
+      for (; k < e; ++k) visit(k);
+      k = kn;
+      e = en;
     }
   }
 }
