@@ -305,19 +305,20 @@ def serving_leg(C, b, rate, n_req, batched=True):
             "budget_bytes": 16 << 30, "max_inflight": 2 if batched else 1}
 
 
-PIPE_POINTS = 8 << 20  # sub-batch size of the library's pipelined host-memory path
+PIPE_POINTS = 8 << 20  # largest sub-batch of the library's pipelined host-memory path (else a sixth of the batch)
 
 
 def copy_floor(torch, off, hin, hout, dev_in, reps=3):
     """The e2e step's copies alone, with no kernels: the same arrays in the
-    same event-aligned sub-batches of about PIPE_POINTS points as the
+    same event-aligned sub-batches as the
     pipelined path (inputs on one stream, outputs on another, overlapped), and
     the same bytes as one copy per array.  The pipelined e2e step cannot beat
     the first; the host link's shared bandwidth sets both."""
     E = len(off) - 1
+    piece = min(PIPE_POINTS, int(off[-1]) // 6)
     cut = [0]
     for e in range(E):
-        if off[e + 1] - off[cut[-1]] >= PIPE_POINTS and e + 1 < E:
+        if off[e + 1] - off[cut[-1]] >= piece and e + 1 < E:
             cut.append(e + 1)
     cut.append(E)
     dev_out = {k: torch.empty(v.numel(), dtype=v.dtype, device="cuda") for k, v in hout.items()}
