@@ -127,12 +127,28 @@ __global__ void __launch_bounds__(kBridgeThreads) k_bridge_count(int64_t N, cons
 }
 
 // The sums of a cluster are exact integers, so they may be added in any
-// grouping: each thread takes kRun consecutive points (read 4 at a time with
-// 16-byte loads), keeps running sums while the cluster stays the same (a
+// grouping: each thread takes kRun consecutive points (read 8 at a time with
+// 32-byte loads), keeps running sums while the cluster stays the same (a
 // cluster's points are mostly consecutive), and makes the three atomic
 // additions once per run.
 constexpr int kRun = kBridgeChunk / kBridgeThreads;  // 16 points per thread
-static_assert(kRun % 4 == 0, "vector loads");
+static_assert(kRun % 8 == 0, "vector loads");
+
+// Eight consecutive words: one 32-byte load, or two of 16 bytes.
+template <class T>
+__device__ __forceinline__ void load8(const T* p, bool wide, T* v) {
+  static_assert(sizeof(T) == 4, "words");
+  unsigned u[8];
+  if (wide) {
+    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "l"(p));
+  } else {
+    const uint4 a = *reinterpret_cast<const uint4*>(p), b = *reinterpret_cast<const uint4*>(p + 4);
+    u[0] = a.x, u[1] = a.y, u[2] = a.z, u[3] = a.w, u[4] = b.x, u[5] = b.y, u[6] = b.z, u[7] = b.w;
+  }
+  memcpy(v, u, 32);
+}
 
 __global__ void __launch_bounds__(kBridgeThreads) k_bridge_accumulate(
     int64_t N, const int64_t* __restrict__ off, const int32_t* __restrict__ chunk_ev,
@@ -172,26 +188,28 @@ __global__ void __launch_bounds__(kBridgeThreads) k_bridge_accumulate(
       if (sd) seed_of[cbase + c] = (int32_t)i;
     }
   };
-  // 16-byte loads when the run is whole, in one event and every array is
-  // 16-byte aligned (i0 is a multiple of 16 points); otherwise points are read
-  // one by one
-  const bool vec = i0 + kRun <= next && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) |
-                                         reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(seed) |
-                                         reinterpret_cast<uintptr_t>(ci)) & 15) == 0;
-  if (vec) {
-    // unrolled, so that the loads of later groups of four are issued before the
-    // earlier groups' fixed-point work (1,000 HGCAL events: 5.74 -> 5.48 ms)
+  // wide loads when the run is whole, in one event and every array is 16-byte
+  // aligned (i0 is a multiple of 16 points); otherwise points are read one by
+  // one.  A thread's run is 64 bytes of each array, so a 16-byte load uses half
+  // of each sector it touches; with 32-byte loads, in groups of eight that are
+  // not unrolled (72 registers when they are), the bridge on 200 HGCAL events
+  // takes 0.49 ms against 0.525.  Arrays on a 16-byte boundary only: 0.515.
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) |
+                       reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(seed) |
+                       reinterpret_cast<uintptr_t>(ci);
+  if (i0 + kRun <= next && (at & 15) == 0) {
+    const bool wide = (at & 31) == 0;
+#pragma unroll 1
+    for (int k0 = 0; k0 < kRun; k0 += 8) {
+      int32_t c8[8], s8[8];
+      float w8[8], x8[8], y8[8];
+      load8(ci + i0 + k0, wide, c8);
+      load8(seed + i0 + k0, wide, s8);
+      load8(w + i0 + k0, wide, w8);
+      load8(x + i0 + k0, wide, x8);
+      load8(y + i0 + k0, wide, y8);
 #pragma unroll
-    for (int k0 = 0; k0 < kRun; k0 += 4) {
-      const int4 c4 = *reinterpret_cast<const int4*>(ci + i0 + k0);
-      const int4 s4 = *reinterpret_cast<const int4*>(seed + i0 + k0);
-      const float4 w4 = *reinterpret_cast<const float4*>(w + i0 + k0);
-      const float4 x4 = *reinterpret_cast<const float4*>(x + i0 + k0);
-      const float4 y4 = *reinterpret_cast<const float4*>(y + i0 + k0);
-      point(c4.x, s4.x, w4.x, x4.x, y4.x, i0 + k0);
-      point(c4.y, s4.y, w4.y, x4.y, y4.y, i0 + k0 + 1);
-      point(c4.z, s4.z, w4.z, x4.z, y4.z, i0 + k0 + 2);
-      point(c4.w, s4.w, w4.w, x4.w, y4.w, i0 + k0 + 3);
+      for (int k = 0; k < 8; ++k) point(c8[k], s8[k], w8[k], x8[k], y8[k], i0 + k0 + k);
     }
   } else {
 #pragma unroll 1

@@ -105,3 +105,32 @@ def test_cluster_fields_over_their_ranges(cuda_lib, place):
             assert max_ulp(got[k], v) <= 1, k
         else:
             assert np.array_equal(got[k].view(np.int32), np.asarray(v).view(np.int32)), k
+
+
+@pytest.mark.parametrize("shift", [8, 4, 1], ids=["32-byte", "16-byte", "4-byte"])
+def test_alignments_of_the_inputs(cuda_lib, shift):
+    """Arrays that start on a 32-byte, a 16-byte and a 4-byte boundary: each has
+    its own loads."""
+    import torch
+    rng = np.random.default_rng(shift)
+    off = np.array([0, 33, 8200], np.int64)
+    n = int(off[-1])
+    w, x = _values("heavy", rng, n)
+    _, y = _values("edges", rng, n)
+    local = np.concatenate([np.arange(s) for s in np.diff(off)])
+    ci = (local // 5).astype(np.int32)
+    seed = (local % 5 == 0).astype(np.int32)
+    layer = (local % 100).astype(np.int32)
+    want_off, want = OB.layer_clusters(off, x, y, layer, w, seed, ci, S.layer_z())
+    d = [torch.from_numpy(np.concatenate([np.zeros(shift, v.dtype), v])).cuda()[shift:]
+         for v in (x, y, layer, w, seed, ci)]
+    algo = C.Clusterizer(1.3, 2.0, 2.0)
+    got_off, got = algo.layer_clusters(off, *d[:4], dict(isSeed=d[4], clusterIndex=d[5]))
+    got = {k: v.cpu().numpy() for k, v in got.items()}
+    algo.close()
+    assert np.array_equal(got_off, want_off)
+    for k, v in want.items():
+        if k in ("eta", "phi"):
+            assert max_ulp(got[k], v) <= 1, k
+        else:
+            assert np.array_equal(got[k].view(np.int32), np.asarray(v).view(np.int32)), k
