@@ -1001,19 +1001,24 @@ __global__ void __launch_bounds__(256) k_seed_rank(Batch2D b) {
 
 // kHostOut: a small host run, whose outputs also go to the page-locked staging
 // (an instantiation of its own: the branch cost the others 0.1 ms per 65M points).
+// There a chunk is cut into slices of a block each: a block's stores to host
+// memory complete a few at a time, and a 5,000-point event is two chunks (one
+// host call of 5,000 points: 67 -> 58 us; this kernel 21.8 -> 5.6 us).
+constexpr int kHostSlices = 8;
 template <bool kHostOut>
 __global__ void __launch_bounds__(kChunkThreads) k_label(Batch2D b) {
-  const int c = blockIdx.x;
+  constexpr int kSlices = kHostOut ? kHostSlices : 1;
+  const int c = blockIdx.x / kSlices;
   __shared__ int s_e;
   pdl_wait();
   // the run's status words, final by now, to the host's page-locked copy
-  if (c == 0 && threadIdx.x < kFlagCount && b.host_flags) b.host_flags[threadIdx.x] = b.flags[threadIdx.x];
+  if (blockIdx.x == 0 && threadIdx.x < kFlagCount && b.host_flags) b.host_flags[threadIdx.x] = b.flags[threadIdx.x];
   if (threadIdx.x == 0) s_e = event_of_chunk(b, c);
   __syncthreads();
   const int e = s_e;
   const int64_t es = b.offsets[e], ee = b.offsets[e + 1];
-  const int64_t i0 = es + (int64_t)(c - b.chunk_start[e]) * kChunk;
-  const int64_t i1 = min(i0 + (int64_t)kChunk, ee);
+  const int64_t i0 = es + (int64_t)(c - b.chunk_start[e]) * kChunk + blockIdx.x % kSlices * (kChunk / kSlices);
+  const int64_t i1 = min(i0 + kChunk / kSlices, ee);
   const int64_t n_ev = ee - es;
   // ci holds a seed's rank (>= 0, from k_seed_rank), -1 (no cluster), or
   // -(root + 2) for a point whose chain ends at the seed `root` (event-local
@@ -1021,7 +1026,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_label(Batch2D b) {
   // with an invalid layer were never written, so the root is range-checked.
   // The roots are seeds, which this kernel never writes; the gathers of one
   // thread's points are issued together.
-  constexpr int PER = kChunk / kChunkThreads;
+  constexpr int PER = kChunk / kSlices / kChunkThreads;
   int v[PER], r[PER];
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
@@ -1311,7 +1316,7 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
   mark(6);
   {
     NvtxRange r("clue2d/label");
-    err = b.host_out ? launch_pdl(k_label<true>, nc, kChunkThreads, 0, s, b)
+    err = b.host_out ? launch_pdl(k_label<true>, nc * kHostSlices, kChunkThreads, 0, s, b)
                      : launch_pdl(k_label<false>, nc, kChunkThreads, 0, s, b);
     if (err != cudaSuccess) return err;
   }
