@@ -814,6 +814,11 @@ __global__ void __launch_bounds__(kSizeBuckets) k_order(Batch2D b) {
 // the index order).  With a global atomic per warp group of every pass the
 // passes ran one after another at its round trip: 57 -> 21 us on one shuffled
 // HGCAL event of 323k points.
+// kSlices blocks per chunk where the chunks are fewer than the SMs (the kernel
+// then waits on each block's chain of rank, reservation and stores): the same
+// event as a host call 275 -> 270 us with four; with more chunks one block
+// each, which reserves and adds less.
+template <int kSlices>
 __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
   __shared__ int s_e;
   __shared__ int s_cnt[kLayers];  // the chunk's points per layer, then the position of the first
@@ -821,15 +826,16 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
   const unsigned lt = (1u << lane) - 1u;
   pdl_begin();
   if (b.flags[kFlagGrouped]) return;  // input already grouped by layer
-  for (int c = blockIdx.x; c < b.n_chunks; c += gridDim.x) {
+  for (int it = blockIdx.x; it < b.n_chunks * kSlices; it += gridDim.x) {
+    const int c = it / kSlices;
     for (int l = threadIdx.x; l < kLayers; l += kChunkThreads) s_cnt[l] = 0;
     if (threadIdx.x == 0) s_e = event_of_chunk(b, c);
     __syncthreads();
     const int e = s_e;
     const int64_t es = b.offsets[e], ee = b.offsets[e + 1];
-    const int64_t i0 = es + (int64_t)(c - b.chunk_start[e]) * kChunk;
-    const int64_t i1 = min(i0 + (int64_t)kChunk, ee);
-    constexpr int PER = kChunk / kChunkThreads;
+    const int64_t i0 = es + (int64_t)(c - b.chunk_start[e]) * kChunk + it % kSlices * (kChunk / kSlices);
+    const int64_t i1 = min(i0 + kChunk / kSlices, ee);
+    constexpr int PER = kChunk / kSlices / kChunkThreads;
     int lv[PER], rank[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
@@ -1109,7 +1115,8 @@ cudaError_t prepare_clue2d_kernels(int device) {
   // later launch of the pipeline has code to load.
   const void* rest[] = {reinterpret_cast<const void*>(k_init), reinterpret_cast<const void*>(k_count),
                         reinterpret_cast<const void*>(k_layer_scan), reinterpret_cast<const void*>(k_order),
-                        reinterpret_cast<const void*>(k_scatter), reinterpret_cast<const void*>(k_seed_chunk_scan),
+                        reinterpret_cast<const void*>(k_scatter<1>), reinterpret_cast<const void*>(k_scatter<4>),
+                        reinterpret_cast<const void*>(k_seed_chunk_scan),
                         reinterpret_cast<const void*>(k_seed_rank), reinterpret_cast<const void*>(k_label<false>),
                         reinterpret_cast<const void*>(k_label<true>)};
   for (const void* f : rest) {
@@ -1260,7 +1267,9 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
     NvtxRange r("clue2d/scatter");
     // a resident grid: grouped input has nothing to do here (57 -> 4 us on the
     // 4096-event batch against a block per chunk)
-    if ((err = launch_pdl(k_scatter, std::min(nc, 152 * 4), kChunkThreads, 0, s, b)) != cudaSuccess) return err;
+    err = nc <= 152 ? launch_pdl(k_scatter<4>, nc * 4, kChunkThreads, 0, s, b)
+                    : launch_pdl(k_scatter<1>, std::min(nc, 152 * 4), kChunkThreads, 0, s, b);
+    if (err != cudaSuccess) return err;
   }
   mark(3);
   // Invariant: every layer-kernel grid is at most n_items = n_events * kLayers

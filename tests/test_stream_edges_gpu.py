@@ -55,6 +55,21 @@ def test_chunk_and_load_edges(cuda_lib, shift, decrease):
     assert_bitexact({k: v.cpu().numpy() for k, v in out.items()}, want)
 
 
+@pytest.mark.parametrize("n", [1023, 1025, 5121, 152 * 4096, 152 * 4096 + 1])
+def test_shuffled_event_sizes(cuda_lib, n):
+    """One event with its layers interleaved, around the slices of a chunk that
+    a block of the grouping kernel takes, and on both sides of 152 chunks."""
+    rng = np.random.default_rng(n)
+    side = 30 + n ** 0.5 / 8
+    x, y = (rng.uniform(-min(side, 200), min(side, 200), n).astype(np.float32) for _ in range(2))
+    layer = rng.integers(0, 100, n).astype(np.int32)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    algo = C.Clusterizer(*PRM)
+    got = algo.make_clusters(x, y, layer, w)
+    algo.close()
+    assert_bitexact(got, oracle.clue2d(x, y, layer, w, *PRM))
+
+
 @pytest.mark.parametrize("n", [1, 31, 4096, 32767, 32768, 32769])
 def test_small_host_runs_and_the_rule(cuda_lib, n):
     """Host-memory runs on both sides of the staging limit (32,768 points),
