@@ -46,3 +46,25 @@ def test_rows(cuda_lib, kind, siblings):
     want, nt = oracle.clue3d(ev, **prm)
     assert int(nts[0]) == nt
     assert_bitexact({NAMES[k]: v for k, v in out.items()}, want, keys=tuple(NAMES.values()), label=kind)
+
+
+@pytest.mark.parametrize("siblings", [2, 3])
+@pytest.mark.parametrize("kind,n", [("row", 6000), ("row", 16000), ("column", 6000), ("column", 2000)])
+def test_crowded_rows(cuda_lib, kind, n, siblings):
+    """Rows searched by their entries' columns, within the room that a slab has
+    for staged columns and beyond it: every cluster of a layer in its first eta row
+    (16,000 clusters: more columns than fit), or in one phi column (more such rows
+    than fit), some of them at the wrap."""
+    ev = S.clue3d_event(11, n_clusters=n, n_layers=94)
+    rng = np.random.default_rng(n)
+    if kind == "row":
+        ev["eta"] = np.minimum(ev["eta"], np.float32(1.4999))
+    else:
+        ev["phi"] = rng.uniform(3.12, math.pi, n).astype(np.float32) * rng.choice([-1, 1], n).astype(np.float32)
+    prm = dict(n_layers=94, density_sibling_layers=siblings, nh_sibling_layers=siblings)
+    algo = C.Clusterizer(1.3, 2.0, 2.0)
+    out, nts = algo.run_clue3d(np.array([0, n], np.int64), ev, params=prm)
+    algo.close()
+    want, nt = oracle.clue3d(ev, **prm)
+    assert int(nts[0]) == nt
+    assert_bitexact({NAMES[k]: v for k, v in out.items()}, want, keys=tuple(NAMES.values()), label=kind)
