@@ -343,34 +343,35 @@ struct RowsStaged {
   __device__ __forceinline__ int col(int q) const { return bins_col(__float_as_int(recs[2 * (int64_t)q + 1].w)); }
 };
 
+// First of the positions [s, t), which are in column order, whose column is at
+// or above a.
+template <class F>
+__device__ __forceinline__ int first_at(int s, int t, int a, F&& col) {
+  int len = t - s;
+  while (len > 0) {
+    const int h = len >> 1;
+    const bool below = col(s + h) < a;
+    s = below ? s + h + 1 : s;
+    len = below ? len - h - 1 : h;
+  }
+  return s;
+}
+
 // Visits the entries of rows [s, t) whose phi column lies in the window
 // [p0, p1] (p0 may be negative, p1 may exceed 125), in the reference's
 // order: iphi_it = p0..p1 mapped modulo 126.
+// The first column is found by a binary search: slabs beyond the staging area
+// walk their rows in global memory (10 events of 100,000 clusters, 31 to a row:
+// 8.9 ms counting from each row's start, 2.3 ms).
 template <class V, class F>
 __device__ __forceinline__ void visit_row(const V& v, int s, int t, int p0, int p1, F&& f) {
-  if (p0 >= 0 && p1 < kPhiBins) {
-    for (int q = s; q < t; ++q) {
-      const int c = v.col(q);
-      if (c > p1) break;
-      if (c >= p0) f(q);
-    }
-    return;
-  }
-  int a0, a1, c0, c1;  // first arc [a0, a1], then [c0, c1]
-  if (p0 < 0) {
-    a0 = p0 + kPhiBins; a1 = kPhiBins - 1; c0 = 0; c1 = p1;
-  } else {
-    a0 = p0; a1 = kPhiBins - 1; c0 = 0; c1 = p1 - kPhiBins;
-  }
-  for (int q = s; q < t; ++q) {
-    const int c = v.col(q);
-    if (c >= a0 && c <= a1) f(q);
-  }
-  for (int q = s; q < t; ++q) {
-    const int c = v.col(q);
-    if (c > c1) break;
-    if (c >= c0) f(q);
-  }
+  const bool wraps = p0 < 0 || p1 >= kPhiBins;
+  const int a0 = p0 < 0 ? p0 + kPhiBins : p0;  // first arc [a0, a1], then [0, c1] when the window wraps
+  const int a1 = wraps ? kPhiBins - 1 : p1;
+  for (int q = first_at(s, t, a0, [&](int k) { return v.col(k); }); q < t && v.col(q) <= a1; ++q) f(q);
+  if (!wraps) return;
+  const int c1 = p0 < 0 ? p1 : p1 - kPhiBins;
+  for (int q = s; q < t && v.col(q) <= c1; ++q) f(q);
 }
 
 // Phi columns of the window [pb - d, pb + d] modulo 126 as a 126-bit mask
@@ -578,17 +579,10 @@ __device__ __forceinline__ RowRuns row_runs(const RowsStaged& v, int r, const Ph
       const int a0 = 32 * f.word + f.sh, a1 = a0 + (f.all == 31u ? 5 : (f.all == 7u ? 3 : 1));
       const uint8_t* cs = v.cols + 4 * ((rs >> kRowStartBits) & ((1 << kRowSlotBits) - 1)) - o.s;
       auto col = [&](int q) { return (rs & kRowCols) ? (int)cs[q] : v.col(q); };
-      int lo = o.s, len = t - o.s;  // first entry in column a0 or above
-      while (len > 0) {
-        const int h = len >> 1;
-        const bool below = col(lo + h) < a0;
-        lo = below ? lo + h + 1 : lo;
-        len = below ? len - h - 1 : h;
-      }
-      o.qa = lo;
-      int q = lo;
+      o.qa = first_at(o.s, t, a0, col);
+      int q = o.qa;
       while (q < t && col(q) < a1) ++q;
-      o.na = q - lo;
+      o.na = q - o.qa;
       q = o.s;
       while (q < t && col(q) < a1 - kPhiBins) ++q;
       o.nb = q - o.s;

@@ -49,17 +49,19 @@ def test_rows(cuda_lib, kind, siblings):
 
 
 @pytest.mark.parametrize("siblings", [2, 3])
-@pytest.mark.parametrize("kind,n", [("row", 6000), ("row", 16000), ("column", 6000), ("column", 2000)])
+@pytest.mark.parametrize("kind,n", [("row", 6000), ("row", 16000), ("column", 6000), ("column", 2000),
+                                    ("wide", 60000), ("row", 40000)])
 def test_crowded_rows(cuda_lib, kind, n, siblings):
     """Rows searched by their entries' columns, within the room that a slab has
     for staged columns and beyond it: every cluster of a layer in its first eta row
     (16,000 clusters: more columns than fit), or in one phi column (more such rows
-    than fit), some of them at the wrap."""
+    than fit), some of them at the wrap; and events whose slabs are searched in
+    global memory, where most rows repeat a column."""
     ev = S.clue3d_event(11, n_clusters=n, n_layers=94)
     rng = np.random.default_rng(n)
     if kind == "row":
         ev["eta"] = np.minimum(ev["eta"], np.float32(1.4999))
-    else:
+    elif kind == "column":
         ev["phi"] = rng.uniform(3.12, math.pi, n).astype(np.float32) * rng.choice([-1, 1], n).astype(np.float32)
     prm = dict(n_layers=94, density_sibling_layers=siblings, nh_sibling_layers=siblings)
     algo = C.Clusterizer(1.3, 2.0, 2.0)
