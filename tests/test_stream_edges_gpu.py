@@ -70,6 +70,24 @@ def test_shuffled_event_sizes(cuda_lib, n):
     assert_bitexact(got, oracle.clue2d(x, y, layer, w, *PRM))
 
 
+@pytest.mark.parametrize("points", [12 << 20, (12 << 20) + 1])
+def test_large_shuffled_batches(cuda_lib, points):
+    """A shuffled batch on both sides of the size from which its layers are
+    taken event by event, with layers of both size classes and an empty event."""
+    rng = np.random.default_rng(points)
+    sizes = rng.integers(20000, 260000, 90)
+    sizes = np.concatenate([[0], (sizes * ((points - 300000) / sizes.sum())).astype(np.int64)])
+    sizes = np.concatenate([sizes, [points - sizes.sum()]])
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    x, y = (rng.uniform(-240, 240, points).astype(np.float32) for _ in range(2))
+    layer = rng.integers(0, 100, points).astype(np.int32)
+    w = rng.exponential(1.0, points).astype(np.float32)
+    algo = C.Clusterizer(*PRM)
+    got = algo.run_batch(off, x, y, layer, w)
+    algo.close()
+    assert_bitexact(got, oracle.clue2d_batch(off, x, y, layer, w, *PRM, n_threads=8))
+
+
 @pytest.mark.parametrize("n", [1, 31, 4096, 32767, 32768, 32769])
 def test_small_host_runs_and_the_rule(cuda_lib, n):
     """Host-memory runs on both sides of the staging limit (32,768 points),
