@@ -836,14 +836,28 @@ __global__ void __launch_bounds__(kSizeBuckets) k_order(Batch2D b) {
 // the index order).  With a global atomic per warp group of every pass the
 // passes ran one after another at its round trip: 57 -> 21 us on one shuffled
 // HGCAL event of 323k points.
-// kSlices blocks per chunk where the chunks are fewer than the SMs (the kernel
-// then waits on each block's chain of rank, reservation and stores): the same
-// event as a host call 275 -> 270 us with four; with more chunks one block
-// each, which reserves and adds less.
+// The chunk is put into layer order in shared memory and stored from there, so
+// that a warp stores runs of a layer's points (some forty of a chunk's) and not 32
+// words in 32 sectors of each array, which bound the kernel (15.4M shuffled points:
+// 0.455 ms, the batch 2.02 -> 1.76 ms; 32M points in 100 HGCAL events 4.15 -> 3.55).
+// (40 registers instead of 64 for three blocks per SM: the same.)  kSlices blocks per chunk where the chunks are fewer than the
+// SMs (the kernel then waits on each block's chain of rank, reservation and
+// stores): a shuffled HGCAL event as a host call 275 -> 270 us with four,
+// 265 with the stores in runs; with
+// more chunks one block each, which reserves and adds less.
+template <int kSlices>
+constexpr size_t kScatterSmem = 17 * (size_t)(kChunk / kSlices);  // a record and a layer per point
+
 template <int kSlices>
 __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  uint4* s_rec = reinterpret_cast<uint4*>(dsm);
+  uint8_t* s_layer = reinterpret_cast<uint8_t*>(s_rec + kChunk / kSlices);
   __shared__ int s_e;
-  __shared__ int s_cnt[kLayers];  // the chunk's points per layer, then the position of the first
+  __shared__ int s_cnt[kLayers];   // the slice's points per layer
+  __shared__ int s_at[kLayers];    // their first slot here
+  __shared__ int s_base[kLayers];  // their first position
+  __shared__ int s_total;
   const int lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
   pdl_begin();
@@ -859,11 +873,18 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
     const int64_t i1 = min(i0 + kChunk / kSlices, ee);
     constexpr int PER = kChunk / kSlices / kChunkThreads;
     int lv[PER], rank[PER];
+    float px[PER], py[PER], pw[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
-      lv[j] = i < i1 ? b.layer[i] : -1;
-      if (lv[j] >= kLayers) lv[j] = -1;
+      lv[j] = -1;
+      if (i < i1) {
+        lv[j] = b.layer[i];
+        px[j] = b.x[i];
+        py[j] = b.y[i];
+        pw[j] = b.w[i];
+        if (lv[j] >= kLayers) lv[j] = -1;
+      }
     }
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
@@ -874,21 +895,55 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
       rank[j] = __shfl_sync(0xffffffffu, old, leader) + __popc(mask & lt);
     }
     __syncthreads();
-    for (int l = threadIdx.x; l < kLayers; l += kChunkThreads)
-      if (s_cnt[l]) s_cnt[l] = atomicAdd(&b.cursor[e * kLayers + l], s_cnt[l]);
+    if (threadIdx.x < 32) {  // slots of the layers, four per lane
+      int n[4], sum = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        n[k] = 4 * lane + k < kLayers ? s_cnt[4 * lane + k] : 0;
+        sum += n[k];
+      }
+      int x = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += t;
+      }
+      if (lane == 31) s_total = x;
+      x -= sum;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (4 * lane + k < kLayers) s_at[4 * lane + k] = x;
+        x += n[k];
+      }
+    } else if (threadIdx.x < 32 + kLayers) {
+      const int l = threadIdx.x - 32;
+      s_base[l] = s_cnt[l] ? atomicAdd(&b.cursor[e * kLayers + l], s_cnt[l]) : 0;
+    }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
-      const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
       if (lv[j] >= 0) {
-        const int pos = s_cnt[lv[j]] + rank[j];
-        b.gx[pos] = b.x[i];
-        b.gy[pos] = b.y[i];
-        b.gw[pos] = b.w[i];
-        b.gid[pos] = (int32_t)(i - es);
+        const int slot = s_at[lv[j]] + rank[j];
+        const int64_t i = i0 + threadIdx.x + (int64_t)j * kChunkThreads;
+        s_rec[slot] = make_uint4(__float_as_uint(px[j]), __float_as_uint(py[j]), __float_as_uint(pw[j]), (unsigned)(i - es));
+        s_layer[slot] = (uint8_t)lv[j];
       }
     }
-    __syncthreads();  // s_cnt of the next chunk
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int slot = threadIdx.x + j * kChunkThreads;
+      if (slot < s_total) {
+        const int l = s_layer[slot];
+        const int pos = s_base[l] + slot - s_at[l];
+        const uint4 r = s_rec[slot];
+        b.gx[pos] = __uint_as_float(r.x);
+        b.gy[pos] = __uint_as_float(r.y);
+        b.gw[pos] = __uint_as_float(r.z);
+        b.gid[pos] = (int32_t)r.w;
+      }
+    }
+    __syncthreads();  // the shared arrays of the next slice
   }
 }
 
@@ -1141,6 +1196,9 @@ cudaError_t prepare_clue2d_kernels(int device) {
                         reinterpret_cast<const void*>(k_seed_chunk_scan),
                         reinterpret_cast<const void*>(k_seed_rank), reinterpret_cast<const void*>(k_label<false>),
                         reinterpret_cast<const void*>(k_label<true>)};
+  if ((e = cudaFuncSetAttribute(k_scatter<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScatterSmem<1>)) !=
+      cudaSuccess)
+    return e;
   for (const void* f : rest) {
     cudaFuncAttributes a;
     if ((e = cudaFuncGetAttributes(&a, f)) != cudaSuccess) return e;
@@ -1289,8 +1347,8 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
     NvtxRange r("clue2d/scatter");
     // a resident grid: grouped input has nothing to do here (57 -> 4 us on the
     // 4096-event batch against a block per chunk)
-    err = nc <= 152 ? launch_pdl(k_scatter<4>, nc * 4, kChunkThreads, 0, s, b)
-                    : launch_pdl(k_scatter<1>, std::min(nc, 152 * 4), kChunkThreads, 0, s, b);
+    err = nc <= 152 ? launch_pdl(k_scatter<4>, nc * 4, kChunkThreads, kScatterSmem<4>, s, b)
+                    : launch_pdl(k_scatter<1>, std::min(nc, 152 * 3), kChunkThreads, kScatterSmem<1>, s, b);
     if (err != cudaSuccess) return err;
   }
   mark(3);
