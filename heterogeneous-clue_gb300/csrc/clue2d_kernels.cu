@@ -839,12 +839,12 @@ __global__ void __launch_bounds__(kSizeBuckets) k_order(Batch2D b) {
 // The chunk is put into layer order in shared memory and stored from there, so
 // that a warp stores runs of a layer's points (some forty of a chunk's) and not 32
 // words in 32 sectors of each array, which bound the kernel (15.4M shuffled points:
-// 0.455 ms, the batch 2.02 -> 1.76 ms; 32M points in 100 HGCAL events 4.15 -> 3.55).
-// (40 registers instead of 64 for three blocks per SM: the same.)  kSlices blocks per chunk where the chunks are fewer than the
-// SMs (the kernel then waits on each block's chain of rank, reservation and
-// stores): a shuffled HGCAL event as a host call 275 -> 270 us with four,
-// 265 with the stores in runs; with
-// more chunks one block each, which reserves and adds less.
+// 0.455 ms, the batch 2.02 -> 1.76 ms; 32M points in 100 HGCAL events 4.15 -> 3.55;
+// 40 registers instead of 64 for three blocks per SM: the same).
+// kSlices blocks per chunk where the chunks are fewer than the SMs (the kernel
+// then waits on each block's chain of rank, reservation and stores): a shuffled
+// HGCAL event as a host call 275 -> 270 us with four, 265 with the stores in
+// runs; with more chunks one block each, which reserves and adds less.
 template <int kSlices>
 constexpr size_t kScatterSmem = 17 * (size_t)(kChunk / kSlices);  // a record and a layer per point
 

@@ -692,7 +692,7 @@ static_assert(kSlabMaxCand < 1 << kRowStartBits && kSlabSlots <= 1 << kRowSlotBi
 constexpr size_t kSlabSmem = 16 * (size_t)kSlabMaxCand + 16 * (size_t)kSlabMaxRows + 16 * (size_t)kSlabSlots +
                              8 * (size_t)(kSlabMaxRows + 1) + 4 * (size_t)kSlabColWords;
 
-template <bool kDensity>
+template <bool kDensity, bool kParts>
 __global__ void __launch_bounds__(kSlabThreads, 5) k3_search(Batch3D b, Params3D P, int n_slabs) {
   extern __shared__ __align__(16) unsigned char sm3[];
   float4* s_cand = reinterpret_cast<float4*>(sm3);
@@ -712,129 +712,148 @@ __global__ void __launch_bounds__(kSlabThreads, 5) k3_search(Batch3D b, Params3D
   const int R = b.n_rows;
   const int64_t rbase = (int64_t)e * R;
   const int32_t* rs = b.row_start + rbase;
-  const int q_lo = rs[L0 * kEtaBins], q_hi = rs[L1 * kEtaBins];
-  if (q_lo >= q_hi) return;
-  // rows of layers [L0 - sib, L1 + sib) and the first row after them (the
-  // reference's eta window reaches row 34 of a layer, the next layer's row 0)
-  const int hl0 = max(L0 - max(sib, 0), 0), hl1 = min(L1 + max(sib, 0), P.n_layers);
-  const int row_lo = hl0 * kEtaBins, row_hi = hl1 * kEtaBins;  // inclusive; row_hi <= R - 2
-  const int nrows = row_hi - row_lo + 1;
-  const int pos_lo = rs[row_lo], pos_hi = rs[row_hi + 1];
-  const bool staged = nrows <= kSlabMaxRows && pos_hi - pos_lo <= kSlabMaxCand;
-  if (staged) {
-    __syncthreads();  // s_slots
-    const uint4* gm = reinterpret_cast<const uint4*>(b.row_mask + 2 * (rbase + row_lo));
-    const uint4* gr = reinterpret_cast<const uint4*>(b.row_rep + 2 * (rbase + row_lo));
-    for (int i = threadIdx.x; i <= nrows; i += kSlabThreads) {
-      int st = rs[row_lo + i] - pos_lo;
-      if (i < nrows) {
-        uint4 m = gm[i], p = make_uint4(0u, 0u, 0u, 0u);
-        if (m.w >> 31) {  // bit 127 of the row's masks: a column repeats / holds a third entry
-          p = gr[i];
-          const int slot = p.w >> 31 ? kSlabSlots : atomicAdd(&s_slots, 1);
-          p.w &= 0x3fffffffu;
-          if (slot < kSlabSlots) {
-            st |= kRowRepeat | (slot << kRowStartBits);
-            reinterpret_cast<uint4*>(s_rep)[slot] = p;
-          } else {
-            const int words = (rs[row_lo + i + 1] - rs[row_lo + i] + 3) >> 2;
-            const int at = atomicAdd(&s_words, words), k = at + words <= kSlabColWords ? atomicAdd(&s_walks, 1) : kSlabWalks;
-            if (k < kSlabWalks) s_walk[k] = i;
-            st |= kRowRepeat | kRowWalk | (k < kSlabWalks ? kRowCols | (at << kRowStartBits) : 0);
-          }
-        }
-        m.w &= 0x3fffffffu;
-        reinterpret_cast<uint4*>(s_mask)[i] = m;
-        const unsigned c0 = __popc(m.x) + __popc(p.x), c1 = c0 + __popc(m.y) + __popc(p.y),
-                       c2 = c1 + __popc(m.z) + __popc(p.z);
-        s_before[i] = (c0 << 8) | (c1 << 16) | (c2 << 24);
+  if (rs[L0 * kEtaBins] >= rs[L1 * kEtaBins]) return;
+  // kParts: the slab in one part, or in halves or single layers where its staging
+  // does not fit (see launch_clue3d)
+  for (int La = L0, Lb; La < L1; La = kParts ? Lb : L1) {
+    // rows of layers [La - sib, Lb + sib) and the first row after them (the
+    // reference's eta window reaches row 34 of a layer, the next layer's row 0)
+    int row_lo, row_hi, nrows, pos_lo, pos_hi;  // row_hi inclusive, <= R - 2
+    bool staged;
+    for (Lb = L1;;) {
+      row_lo = max(La - max(sib, 0), 0) * kEtaBins;
+      row_hi = min(Lb + max(sib, 0), P.n_layers) * kEtaBins;
+      nrows = row_hi - row_lo + 1;
+      pos_lo = rs[row_lo];
+      pos_hi = rs[row_hi + 1];
+      staged = nrows <= kSlabMaxRows && pos_hi - pos_lo <= kSlabMaxCand;
+      if (staged || !kParts) break;
+      if (Lb - La == 1) {  // not even one layer's: from global memory, together
+        Lb = L1;
+        break;
       }
-      s_rs[i] = st;
+      Lb = La + (Lb - La + 1) / 2;
     }
-    for (int i = threadIdx.x; i < pos_hi - pos_lo; i += kSlabThreads) {
-      s_cand[i] = b.rec[2 * (int64_t)(pos_lo + i)];
+    const int q_lo = rs[La * kEtaBins], q_hi = rs[Lb * kEtaBins];
+    if (kParts && La > L0) {
+      __syncthreads();  // the searches of the part before
+      if (threadIdx.x == 0) s_slots = s_walks = s_words = 0;
     }
-    __syncthreads();
-    if (s_walks > 0) {
-      constexpr int kStart = (1 << kRowStartBits) - 1;
-      for (int k = threadIdx.x >> 5; k < min(s_walks, kSlabWalks); k += kSlabThreads / 32) {
-        const int st = s_rs[s_walk[k]], a = st & kStart, z = s_rs[s_walk[k] + 1] & kStart;
-        uint8_t* c = s_col + 4 * ((st >> kRowStartBits) & ((1 << kRowSlotBits) - 1)) - a;
-        for (int q = a + (threadIdx.x & 31); q < z; q += 32)
-          c[q] = (uint8_t)bins_col(__float_as_int(b.rec[2 * (int64_t)(pos_lo + q) + 1].w));
+    if (staged) {
+      __syncthreads();  // s_slots
+      const uint4* gm = reinterpret_cast<const uint4*>(b.row_mask + 2 * (rbase + row_lo));
+      const uint4* gr = reinterpret_cast<const uint4*>(b.row_rep + 2 * (rbase + row_lo));
+      for (int i = threadIdx.x; i <= nrows; i += kSlabThreads) {
+        int st = rs[row_lo + i] - pos_lo;
+        if (i < nrows) {
+          uint4 m = gm[i], p = make_uint4(0u, 0u, 0u, 0u);
+          if (m.w >> 31) {  // bit 127 of the row's masks: a column repeats / holds a third entry
+            p = gr[i];
+            const int slot = p.w >> 31 ? kSlabSlots : atomicAdd(&s_slots, 1);
+            p.w &= 0x3fffffffu;
+            if (slot < kSlabSlots) {
+              st |= kRowRepeat | (slot << kRowStartBits);
+              reinterpret_cast<uint4*>(s_rep)[slot] = p;
+            } else {
+              const int words = (rs[row_lo + i + 1] - rs[row_lo + i] + 3) >> 2;
+              const int at = atomicAdd(&s_words, words), k = at + words <= kSlabColWords ? atomicAdd(&s_walks, 1) : kSlabWalks;
+              if (k < kSlabWalks) s_walk[k] = i;
+              st |= kRowRepeat | kRowWalk | (k < kSlabWalks ? kRowCols | (at << kRowStartBits) : 0);
+            }
+          }
+          m.w &= 0x3fffffffu;
+          reinterpret_cast<uint4*>(s_mask)[i] = m;
+          const unsigned c0 = __popc(m.x) + __popc(p.x), c1 = c0 + __popc(m.y) + __popc(p.y),
+                         c2 = c1 + __popc(m.z) + __popc(p.z);
+          s_before[i] = (c0 << 8) | (c1 << 16) | (c2 << 24);
+        }
+        s_rs[i] = st;
+      }
+      for (int i = threadIdx.x; i < pos_hi - pos_lo; i += kSlabThreads) {
+        s_cand[i] = b.rec[2 * (int64_t)(pos_lo + i)];
       }
       __syncthreads();
+      if (s_walks > 0) {
+        constexpr int kStart = (1 << kRowStartBits) - 1;
+        for (int k = threadIdx.x >> 5; k < min(s_walks, kSlabWalks); k += kSlabThreads / 32) {
+          const int st = s_rs[s_walk[k]], a = st & kStart, z = s_rs[s_walk[k] + 1] & kStart;
+          uint8_t* c = s_col + 4 * ((st >> kRowStartBits) & ((1 << kRowSlotBits) - 1)) - a;
+          for (int q = a + (threadIdx.x & 31); q < z; q += 32)
+            c[q] = (uint8_t)bins_col(__float_as_int(b.rec[2 * (int64_t)(pos_lo + q) + 1].w));
+        }
+        __syncthreads();
+      }
     }
-  }
-  RowsStaged sv{s_mask, s_rep, s_rs, s_before, s_cand, s_col, b.rec + 2 * (int64_t)pos_lo, row_lo};
-  RowsGlobal gv{b.row_mask + 2 * rbase, rs, b.rec};
-  const int64_t es = b.offsets[e];
-  const int tid = threadIdx.x;
-  // the query rows hold only accepted clusters (rejected ones are in the
-  // event's last row); a query's own data is read in sorted order
-  auto query = [&](int p, bool* inside, int* idx) {
-    const float4 qr = b.rec[2 * (int64_t)p + 1];
-    const float4 cr = staged ? s_cand[p - pos_lo] : b.rec[2 * (int64_t)p];
-    *idx = __float_as_int(qr.y);
-    const int bins = __float_as_int(qr.w);
-    Query3 Q;
-    Q.li = bins & 0x7ff;
-    Q.eb = (bins >> 11) & 0x3f;
-    Q.pb = (bins >> 17) & 0x7f;
-    Q.sil = (bins >> 24) & 1;
-    Q.energy = cr.z;
-    Q.phi = cr.y;
-    Q.z = qr.x;
-    Q.r0 = __fmul_rn(cr.x, qr.x);
-    Q.aux = kDensity ? qr.z : cr.w;
-    int lo, hi;
-    layer_window(Q.li, sib, P.n_layers, kDensity ? 0 : 1, &lo, &hi);
-    *inside = staged && lo * kEtaBins >= row_lo && hi * kEtaBins + kEtaBins <= row_hi;
-    Q.self = *inside ? p - pos_lo : p;
-    return Q;
-  };
-  for (int p = q_lo + tid; p < q_hi; p += kSlabThreads) {
-    bool inside;
-    int idx;
-    const Query3 Q = query(p, &inside, &idx);
-    const int64_t gi = es + idx;
-    // staged windows: the rows holding an entry first, in one uniform pass
-    unsigned long long live = 0;
-    bool by_live = false;
-    if (inside) {
-      const Window3 w = window_of(P, Q, kDensity);
-      by_live = live_rows(sv, w.lo, w.hi, w.skip, w.e0, w.e1, PhiField(Q.pb, kDensity ? 2 : 1), &live);
-    }
-    if constexpr (kDensity) {
-      float rho = 0.f;
-      if (by_live) search_live<true>(sv, P, Q, live, rho);
-      else if (inside) search_all<true>(sv, P, Q, rho);
-      else search_all<true>(gv, P, Q, rho);
-      b.rho[gi] = rho;
-      reinterpret_cast<float*>(b.rec)[8 * (int64_t)p + 3] = rho;
-    } else {
-      Nh3 o;
-      if (by_live) search_live<false>(sv, P, Q, live, o);
-      else if (inside) search_all<false>(sv, P, Q, o);
-      else search_all<false>(gv, P, Q, o);
-      if (o.nq >= 0 && inside) o.nq += pos_lo;
-      const bool found = o.best != FLT_MAX;
-      const float dt = found ? o.best_t : FLT_MAX;
-      const int dl = found ? o.best_l : INT_MAX, nl = found ? o.nl : -1;
-      const int ni = found ? __float_as_int(b.rec[2 * (int64_t)o.nq + 1].y) : -1;
-      b.delta_t[gi] = dt;
-      b.delta_l[gi] = dl;
-      b.nh_l[gi] = nl;
-      b.nh_i[gi] = ni;
-      // seeds and outliers (CLUE3DAlgoKernels.h:521-560); par: the nearest
-      // higher for followers, -2 for seeds, -3 for other roots
-      const float r = Q.aux;
-      const float dxy = Q.sil ? P.crit_xy : b.radius[gi];
-      const bool seed = (dt > dxy || __int2float_rn(dl) > P.crit_z) && (r >= P.crit_rho) &&
-                        (__fdiv_rn(Q.energy, r) > P.crit_self);
-      const bool outlier = (dt > P.out_thr) && (r < P.crit_rho);
-      b.seed[gi] = seed ? 1 : 0;
-      b.par[gi] = seed ? -2 : ((!outlier && nl >= 0) ? ni : -3);
+    RowsStaged sv{s_mask, s_rep, s_rs, s_before, s_cand, s_col, b.rec + 2 * (int64_t)pos_lo, row_lo};
+    RowsGlobal gv{b.row_mask + 2 * rbase, rs, b.rec};
+    const int64_t es = b.offsets[e];
+    const int tid = threadIdx.x;
+    // the query rows hold only accepted clusters (rejected ones are in the
+    // event's last row); a query's own data is read in sorted order
+    auto query = [&](int p, bool* inside, int* idx) {
+      const float4 qr = b.rec[2 * (int64_t)p + 1];
+      const float4 cr = staged ? s_cand[p - pos_lo] : b.rec[2 * (int64_t)p];
+      *idx = __float_as_int(qr.y);
+      const int bins = __float_as_int(qr.w);
+      Query3 Q;
+      Q.li = bins & 0x7ff;
+      Q.eb = (bins >> 11) & 0x3f;
+      Q.pb = (bins >> 17) & 0x7f;
+      Q.sil = (bins >> 24) & 1;
+      Q.energy = cr.z;
+      Q.phi = cr.y;
+      Q.z = qr.x;
+      Q.r0 = __fmul_rn(cr.x, qr.x);
+      Q.aux = kDensity ? qr.z : cr.w;
+      int lo, hi;
+      layer_window(Q.li, sib, P.n_layers, kDensity ? 0 : 1, &lo, &hi);
+      *inside = staged && lo * kEtaBins >= row_lo && hi * kEtaBins + kEtaBins <= row_hi;
+      Q.self = *inside ? p - pos_lo : p;
+      return Q;
+    };
+    for (int p = q_lo + tid; p < q_hi; p += kSlabThreads) {
+      bool inside;
+      int idx;
+      const Query3 Q = query(p, &inside, &idx);
+      const int64_t gi = es + idx;
+      // staged windows: the rows holding an entry first, in one uniform pass
+      unsigned long long live = 0;
+      bool by_live = false;
+      if (inside) {
+        const Window3 w = window_of(P, Q, kDensity);
+        by_live = live_rows(sv, w.lo, w.hi, w.skip, w.e0, w.e1, PhiField(Q.pb, kDensity ? 2 : 1), &live);
+      }
+      if constexpr (kDensity) {
+        float rho = 0.f;
+        if (by_live) search_live<true>(sv, P, Q, live, rho);
+        else if (inside) search_all<true>(sv, P, Q, rho);
+        else search_all<true>(gv, P, Q, rho);
+        b.rho[gi] = rho;
+        reinterpret_cast<float*>(b.rec)[8 * (int64_t)p + 3] = rho;
+      } else {
+        Nh3 o;
+        if (by_live) search_live<false>(sv, P, Q, live, o);
+        else if (inside) search_all<false>(sv, P, Q, o);
+        else search_all<false>(gv, P, Q, o);
+        if (o.nq >= 0 && inside) o.nq += pos_lo;
+        const bool found = o.best != FLT_MAX;
+        const float dt = found ? o.best_t : FLT_MAX;
+        const int dl = found ? o.best_l : INT_MAX, nl = found ? o.nl : -1;
+        const int ni = found ? __float_as_int(b.rec[2 * (int64_t)o.nq + 1].y) : -1;
+        b.delta_t[gi] = dt;
+        b.delta_l[gi] = dl;
+        b.nh_l[gi] = nl;
+        b.nh_i[gi] = ni;
+        // seeds and outliers (CLUE3DAlgoKernels.h:521-560); par: the nearest
+        // higher for followers, -2 for seeds, -3 for other roots
+        const float r = Q.aux;
+        const float dxy = Q.sil ? P.crit_xy : b.radius[gi];
+        const bool seed = (dt > dxy || __int2float_rn(dl) > P.crit_z) && (r >= P.crit_rho) &&
+                          (__fdiv_rn(Q.energy, r) > P.crit_self);
+        const bool outlier = (dt > P.out_thr) && (r < P.crit_rho);
+        b.seed[gi] = seed ? 1 : 0;
+        b.par[gi] = seed ? -2 : ((!outlier && nl >= 0) ? ni : -3);
+      }
     }
   }
 }
@@ -943,9 +962,11 @@ __global__ void k3_label(Batch3D b) {
 
 cudaError_t prepare_clue3d_kernels() {
   // more than the 48 KB a kernel may use without asking
-  cudaError_t e = cudaFuncSetAttribute(k3_search<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k3_search<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem);
+  for (auto* k : {k3_search<true, false>, k3_search<true, true>, k3_search<false, false>, k3_search<false, true>}) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_clue3d(const Batch3D& b, const Params3D& p, cudaStream_t s) {
@@ -978,16 +999,29 @@ cudaError_t launch_clue3d(const Batch3D& b, const Params3D& p, cudaStream_t s) {
   const int n_slabs = (p.n_layers + kSlabLayers - 1) / kSlabLayers;
   const int64_t slab_blocks = (int64_t)b.n_events * n_slabs;
   if (slab_blocks > INT32_MAX) return cudaErrorInvalidValue;
+  // Whether the batch's largest event, its clusters spread evenly over the
+  // layers, would fill seven eighths of the staging area (1,792 candidates to a
+  // slab: six standard deviations below its 2,048): such slabs may have to be
+  // searched in parts (100 events of 20,000 clusters with three sibling layers,
+  // 2,130 candidates to a slab: 1.42 ms from global memory, 0.59 in two parts).
+  // Other batches keep the form without the loop (1,000 events of up to 20,000 with
+  // two: 2.07 ms, 2.10 with it); a slab that is crowded all the same then reads
+  // global memory.
+  auto parts = [&](int sib) {
+    return (int64_t)b.max_event * (kSlabLayers + 2 * (int64_t)std::clamp(sib, 0, p.n_layers)) >
+           (int64_t)p.n_layers * (kSlabMaxCand / 8 * 7);
+  };
   {
     NvtxRange r("clue3d/density");
-    if ((err = launch_pdl(k3_search<true>, (unsigned)slab_blocks, kSlabThreads, kSlabSmem, s, b, p, n_slabs)) != cudaSuccess)
-      return err;
+    err = launch_pdl(parts(p.dens_sib) ? k3_search<true, true> : k3_search<true, false>, (unsigned)slab_blocks, kSlabThreads,
+                     kSlabSmem, s, b, p, n_slabs);
+    if (err != cudaSuccess) return err;
   }
   {
     NvtxRange r("clue3d/nearest_higher");
-    if ((err = launch_pdl(k3_search<false>, (unsigned)slab_blocks, kSlabThreads, kSlabSmem, s, b, p, n_slabs)) !=
-        cudaSuccess)
-      return err;
+    err = launch_pdl(parts(p.nh_sib) ? k3_search<false, true> : k3_search<false, false>, (unsigned)slab_blocks, kSlabThreads,
+                     kSlabSmem, s, b, p, n_slabs);
+    if (err != cudaSuccess) return err;
   }
   {
     NvtxRange r("clue3d/finish");

@@ -160,6 +160,7 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     b.host_flags = static_cast<int32_t*>(h->flags_host.p);
     b.offsets = static_cast<const int64_t*>(P(T_TABLES));
     b.blk_ev = b.table_dst + 2 * (size_t)(E + 1);
+    for (int32_t k = 0; k < E; ++k) b.max_event = std::max(b.max_event, off[k + 1] - off[k]);
     const void* din[8];
     void* dout[7];
     const size_t n4 = 4 * (size_t)N;

@@ -70,3 +70,28 @@ def test_crowded_rows(cuda_lib, kind, n, siblings):
     want, nt = oracle.clue3d(ev, **prm)
     assert int(nts[0]) == nt
     assert_bitexact({NAMES[k]: v for k, v in out.items()}, want, keys=tuple(NAMES.values()), label=kind)
+
+
+@pytest.mark.parametrize("layers,siblings,n", [(94, 2, 21056), (94, 2, 21057), (94, 3, 19000), (94, 3, 33000), (10, 2, 3000),
+                                               (7, 3, 1500), (1, 2, 700)])
+def test_slabs_in_parts(cuda_lib, layers, siblings, n):
+    """Slabs around the size from which they may be searched in halves or single
+    layers, with an event beyond it and a crowded layer beside small ones, and layer
+    counts that leave a slab of one to three layers."""
+    rng = np.random.default_rng(n + layers)
+    evs = [S.clue3d_event(21, n_clusters=n, n_layers=max(layers, 2)), S.clue3d_event(22, n_clusters=900, n_layers=max(layers, 2))]
+    for ev in evs:
+        ev["layer"] = np.minimum(ev["layer"], layers - 1).astype(np.int32)
+    crowd = rng.random(n) < 0.1
+    evs[0]["layer"][crowd] = layers // 2
+    off = np.array([0, n, n + 900], np.int64)
+    both = {k: np.concatenate([ev[k] for ev in evs]) for k in evs[0]}
+    prm = dict(n_layers=layers, density_sibling_layers=siblings, nh_sibling_layers=siblings)
+    algo = C.Clusterizer(1.3, 2.0, 2.0)
+    out, nts = algo.run_clue3d(off, both, params=prm)
+    algo.close()
+    for e, ev in enumerate(evs):
+        want, nt = oracle.clue3d(ev, **prm)
+        assert int(nts[e]) == nt
+        assert_bitexact({NAMES[k]: v[off[e]:off[e + 1]] for k, v in out.items()}, want, keys=tuple(NAMES.values()),
+                        label=f"event {e}")
