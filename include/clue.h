@@ -120,7 +120,7 @@ size_t clue_required_bytes(int32_t n_events, int64_t n_points, int flags);
 
 /* Stages of the batched pipeline, in launch order. */
 #define CLUE_N_STAGES 7 /* count, layer_scan (with the largest-first order when taken), scatter,
-                           layers (which also counts seeds per chunk), seed_chunk_scan, seed_rank, label */
+                           layers (which also marks the seeds as bits), seed_chunk_scan, seed_rank, label */
 
 /* Runs one batch like clue_run_batch (device memory, direct launches) and
  * writes each stage's duration in milliseconds to stage_ms[CLUE_N_STAGES],
