@@ -108,6 +108,7 @@ struct Batch2D {
   int32_t* lstart = nullptr;  // [E*100] first grouped position of (event, layer)
   int32_t* cursor = nullptr;  // [E*100]
   int32_t use_order = 0;         // set per launch: take the layers in `order`
+  bool small_layers = false;     // set per launch: small layers are taken by the warp
   int32_t order_big = 0;         // set per launch: size classes of the large-layer pass (0: one class of layers)
   int32_t* order = nullptr;      // [E*100] non-empty (event, layer) items, largest first
   int32_t* size_hist = nullptr;  // [2*kSizeBuckets] layers per size class, then cursors
