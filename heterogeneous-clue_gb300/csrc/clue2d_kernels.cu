@@ -1584,14 +1584,19 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
       // of the large pass run out of layers, instead of after the last one has
       // ended, and the large layers start first, not last (48 uneven events 295
       // -> 261 us; 200 HGCAL events, all of whose layers are large, 5.61 -> 5.58 ms).
+      // With up to three layers per CTA one after the other, large layers first: side
+      // by side their few long layers share SMs to the end (8 events 154 against
+      // 120 us, 12: 159 / 132, 16: 142 / 134; but 24: 178 / 210, 48: 257 / 280).
+      if (n_items <= 3 * grid) side = nullptr;
+      const LaunchKind kind = side ? kOrdinary : kDependent;
       Batch2D large = b;
       large.cursor = b.order;  // the list that the large-layer pass drains
       cudaStream_t s2 = side ? side->stream : s;
       if (side && (err = cudaEventRecord(side->fork, s)) != cudaSuccess) return err;
       err = launch_layers_any(big.threads, large, p, big.layer_capacity, INT_MAX, 1, layer_grid(big, n_items), s,
-                              kOrdinary);
+                              kind);
       if (err == cudaSuccess && side) err = cudaStreamWaitEvent(s2, side->fork, 0);
-      if (err == cudaSuccess) err = launch_layers_any(tt.threads, b, p, tt.layer_capacity, max_m, 0, grid, s2, kOrdinary);
+      if (err == cudaSuccess) err = launch_layers_any(tt.threads, b, p, tt.layer_capacity, max_m, 0, grid, s2, kind);
       if (err == cudaSuccess && side) err = cudaEventRecord(side->join, s2);
       if (err == cudaSuccess && side) err = cudaStreamWaitEvent(s, side->join, 0);
     } else {
