@@ -135,8 +135,7 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     if (rc) return rc;
     const bool staged = host_io && N <= kStagedIoPoints && host_accessible(ins, 8) && host_accessible(outs, 7);
     if (staged) {
-      rc = h->io_stage.reserve(60 * (size_t)N);
-      if (rc) return rc;
+      if ((rc = h->io_stage.reserve(60 * (size_t)N)) || (rc = h->wait_queued())) return rc;
     }
     memcpy(h->stage.p, off, 8 * (size_t)(E + 1));
     // the event of each 256-cluster block's first cluster, so that a kernel

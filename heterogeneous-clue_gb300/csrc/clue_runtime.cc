@@ -232,6 +232,18 @@ int Handle::wait_previous() {
   return CLUE_OK;
 }
 
+// The work queued so far on a caller's stream, before the calling thread itself
+// touches a caller's arrays: a run's inputs are those that its stream's order
+// gives.  On the handle's own stream there is only the handle's work, which
+// wait_previous() has waited for.  (By an event and not by the stream's state: a
+// blocking stream is also ordered behind the default stream's work.)
+int Handle::wait_queued() {
+  if (stream == owned_stream) return CLUE_OK;
+  cudaError_t e = cudaEventRecord(done_event, stream);
+  if (e == cudaSuccess) e = cudaEventSynchronize(done_event);
+  return e == cudaSuccess ? CLUE_OK : cuda_error(e, "waiting for the stream's earlier work");
+}
+
 // The side stream of ordered batches, when this one may be one (outside any
 // stream capture of ours).
 int Handle::ensure_side(int n_events) {
@@ -394,8 +406,7 @@ int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nul
   clue_outputs staged_out;
   if (staged) {
     const size_t n4 = 4 * (size_t)r.N;
-    rc = h->io_stage.reserve(9 * n4);
-    if (rc) return rc;
+    if ((rc = h->io_stage.reserve(9 * n4)) || (rc = h->wait_queued())) return rc;
     char* st = static_cast<char*>(h->io_stage.p);
     for (int i = 0; i < 4; ++i) memcpy(st + i * n4, io[i], n4);
     r.x = reinterpret_cast<const float*>(st);

@@ -105,7 +105,9 @@ constexpr int kAsyncHostIO = 0x100;
 // host copies instead of a stream copy per array (9 or 15 of them, each
 // staged by the driver).  Producer call on 5k / 25k points 105 -> 64 / 143 ->
 // 105 us; at 50k points the host copies cost more (152 -> 163 us).  CLUE3D on
-// 5k layer clusters 168 -> 118 us, on 50k 252 -> 300 us.
+// 5k layer clusters 168 -> 118 us, on 50k 252 -> 300 us.  The calling thread
+// reads the arrays, so on a caller's stream it first waits for the work queued
+// there, which may fill them (Handle::wait_queued).
 constexpr int64_t kStagedIoPoints = int64_t(32) << 10;
 // Whether the CPU may read and write all of these arrays.
 bool host_accessible(const void* const* p, int n);
@@ -143,6 +145,7 @@ struct Handle {
 
   ~Handle();
   int wait_previous();
+  int wait_queued();
   int ensure_side(int n_events);
   int check_device_flags();
   int profile_batch(int32_t E, const int64_t* off, const float* x, const float* y, const int32_t* layer,
