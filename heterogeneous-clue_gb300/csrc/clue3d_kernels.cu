@@ -712,7 +712,10 @@ __global__ void __launch_bounds__(kSlabThreads, 5) k3_search(Batch3D b, Params3D
   const int R = b.n_rows;
   const int64_t rbase = (int64_t)e * R;
   const int32_t* rs = b.row_start + rbase;
-  if (rs[L0 * kEtaBins] >= rs[L1 * kEtaBins]) return;
+  // the last layer's clusters end with the row behind it, which holds those of
+  // phi bin 126 in its last eta row
+  auto layers_end = [&](int l) { return rs[l * kEtaBins + (l == P.n_layers ? 1 : 0)]; };
+  if (rs[L0 * kEtaBins] >= layers_end(L1)) return;
   // kParts: the slab in one part, or in halves or single layers where its staging
   // does not fit (see launch_clue3d)
   for (int La = L0, Lb; La < L1; La = kParts ? Lb : L1) {
@@ -734,7 +737,7 @@ __global__ void __launch_bounds__(kSlabThreads, 5) k3_search(Batch3D b, Params3D
       }
       Lb = La + (Lb - La + 1) / 2;
     }
-    const int q_lo = rs[La * kEtaBins], q_hi = rs[Lb * kEtaBins];
+    const int q_lo = rs[La * kEtaBins], q_hi = layers_end(Lb);
     if (kParts && La > L0) {
       __syncthreads();  // the searches of the part before
       if (threadIdx.x == 0) s_slots = s_walks = s_words = 0;
