@@ -244,12 +244,29 @@ int Handle::wait_queued() {
   return e == cudaSuccess ? CLUE_OK : cuda_error(e, "waiting for the stream's earlier work");
 }
 
+// Priority of a stream (the default where it cannot be told).
+static int priority_of(cudaStream_t s) {
+  int p = 0;
+  if (cudaStreamGetPriority(s, &p) != cudaSuccess) cudaGetLastError();
+  return p;
+}
+
 // The side stream of ordered batches, when this one may be one (outside any
-// stream capture of ours).
+// stream capture of ours), with the priority of the run's stream.
 int Handle::ensure_side(int n_events) {
-  if (side.join || !layers_ordered(tuning, n_events * kLayers)) return CLUE_OK;
-  cudaError_t e = side.stream ? cudaSuccess : cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking);
-  if (e != cudaSuccess) side.stream = nullptr;
+  const int priority = priority_of(stream);
+  if (side_stream() && side_priority == priority) return CLUE_OK;
+  if (!layers_ordered(tuning, n_events * kLayers)) return CLUE_OK;
+  if (side.stream && side_priority != priority) {  // the handle has moved to another stream; no run is pending
+    cudaStreamDestroy(side.stream);
+    side.stream = nullptr;
+  }
+  cudaError_t e = cudaSuccess;
+  if (!side.stream) {
+    e = cudaStreamCreateWithPriority(&side.stream, cudaStreamNonBlocking, priority);
+    if (e != cudaSuccess) side.stream = nullptr;
+    side_priority = priority;
+  }
   for (auto* ev : {&side.fork, &side.join}) {
     if (e != cudaSuccess || *ev) continue;
     if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess) *ev = nullptr;
@@ -311,7 +328,7 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
       return cuda_error(e, "H2D points");
     }
   }
-  e = launch_clue2d(b, h->p2d, h->tuning, s, stage_events, kernels, h->side.join ? &h->side : nullptr);
+  e = launch_clue2d(b, h->p2d, h->tuning, s, stage_events, kernels, h->side_stream());
   if (e != cudaSuccess) return cuda_error(e, "launching CLUE kernels");
   if (host_io && !b.host_out) {
     const clue_outputs* o = r.out;
@@ -459,8 +476,8 @@ int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nul
   cudaError_t e;
   int64_t kernels = 0;
   if (use_graph) {
-    GraphKey key{r.E, r.N, nchunks, h->arena.generation(), r.flags, h->tuning.threads, h->tuning.layer_capacity,
-                 h->tuning.ctas_per_sm,
+    GraphKey key{r.E, r.N, nchunks, h->arena.generation(), r.flags, priority_of(h->stream), h->tuning.threads,
+                 h->tuning.layer_capacity, h->tuning.ctas_per_sm,
                  h->tuning.big_threads, h->tuning.big_capacity,
                  h->tuning.work_tile_cm, h->p2d.dc, h->p2d.rhoc, h->p2d.odf,
                  {(const void*)r.x, (const void*)r.y, (const void*)r.layer, (const void*)r.w,
@@ -700,6 +717,8 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
       return cuda_error(e, "cudaEventCreate");
     }
   }
+  for (int i = 0; i < S; ++i)  // before any copy into or out of the caller's arrays is queued
+    if ((rc = h->ensure_side(cut[i + 1] - cut[i]))) return rc;
   cudaEvent_t* h2d = h->pipe_events;
   cudaEvent_t* comp = h->pipe_events + kPipeSlots;
   cudaEvent_t* d2h = h->pipe_events + 2 * kPipeSlots;
@@ -745,9 +764,7 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
     if ((e = cudaStreamWaitEvent(cs, h2d[k], 0)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(cs, d2h[k], 0)) != cudaSuccess)
       return cuda_error(e, "sub-batch set-up");
-    if ((rc = h->ensure_side(Es))) return rc;
-    if ((e = launch_clue2d(b, h->p2d, h->tuning, cs, nullptr, &kernels, h->side.join ? &h->side : nullptr)) !=
-        cudaSuccess)
+    if ((e = launch_clue2d(b, h->p2d, h->tuning, cs, nullptr, &kernels, h->side_stream())) != cudaSuccess)
       return cuda_error(e, "launching CLUE kernels");
     if ((e = cudaEventRecord(comp[k], cs)) != cudaSuccess) return cuda_error(e, "cudaEventRecord");
     const clue_outputs* o = r.out;

@@ -70,12 +70,14 @@ struct GraphKey {
   int64_t nchunks = -1;     // launch sizes of the chunk kernels are baked into the graph
   uint64_t arena_gen = 0;   // and so are the addresses of every arena buffer
   int flags = 0;
+  int priority = 0;         // of the captured stream: kernel nodes keep it
   int threads = 0, cap = 0, ctas = 0, big_threads = 0, big_cap = 0;
   float work_tile = 0.f;
   float dc = 0.f, rhoc = 0.f, odf = 0.f;
   const void* ptrs[14] = {};
   bool operator==(const GraphKey& o) const {
     if (E != o.E || N != o.N || nchunks != o.nchunks || arena_gen != o.arena_gen || flags != o.flags ||
+        priority != o.priority ||
         threads != o.threads || cap != o.cap || ctas != o.ctas ||
         big_threads != o.big_threads || big_cap != o.big_cap ||
         work_tile != o.work_tile || dc != o.dc || rhoc != o.rhoc || odf != o.odf)
@@ -132,6 +134,7 @@ struct Handle {
   cudaStream_t copy_in = nullptr;         // pipelined host-memory path: H2D stream
   cudaStream_t copy_out = nullptr;        // and D2H stream
   SideStream side;                        // small layers of ordered batches; created by the first of them
+  int side_priority = 0;                  // and its priority, that of the run's stream
   cudaEvent_t pipe_events[3 * kPipeSlots] = {};  // per slot: H2D done, kernels done, D2H done
   clue_run_stats last_run{};              // copies and kernels of the last 2D run
   int64_t graph_kernels = 0;              // kernels in graph_exec
@@ -147,6 +150,7 @@ struct Handle {
   int wait_previous();
   int wait_queued();
   int ensure_side(int n_events);
+  const SideStream* side_stream() const { return side.stream && side.join ? &side : nullptr; }
   int check_device_flags();
   int profile_batch(int32_t E, const int64_t* off, const float* x, const float* y, const int32_t* layer,
                     const float* w, const clue_outputs* out, float* stage_ms);
