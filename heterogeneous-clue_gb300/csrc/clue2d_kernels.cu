@@ -589,7 +589,7 @@ __device__ void process_layer(const Params2D& P, const LayerStore<TT, QT>& S, co
       b.nh[o] = best >= 0 ? (int)S.rec[best].z : -1;
       b.seed[o] = seed ? 1 : 0;
       // the seeds of each event-aligned chunk of 4096 points as bits, for the seed ranks
-      if (seed) atomicOr(&b.seed_bits[(int64_t)in.chunk0 * kChunkWords + (rq.z >> 5)], 1u << (rq.z & 31));
+      if (seed && b.seed_bits) atomicOr(&b.seed_bits[(int64_t)in.chunk0 * kChunkWords + (rq.z >> 5)], 1u << (rq.z & 31));
       par[q] = (!seed && !outlier && best >= 0) ? best : (seed ? -2 : -3);
     }
   }
@@ -770,7 +770,7 @@ __device__ __forceinline__ void tiny_layer(const Params2D& P, unsigned char* ws,
     b.delta[o] = best_s;
     b.nh[o] = best[j] >= 0 ? (int)rec[best[j]].z : -1;
     b.seed[o] = seed ? 1 : 0;
-    if (seed) atomicOr(&b.seed_bits[(int64_t)in.chunk0 * kChunkWords + (gq[j] >> 5)], 1u << (gq[j] & 31));
+    if (seed && b.seed_bits) atomicOr(&b.seed_bits[(int64_t)in.chunk0 * kChunkWords + (gq[j] >> 5)], 1u << (gq[j] & 31));
     nh[q] = (!seed && !outlier && best[j] >= 0) ? best[j] : (seed ? -2 : -3);
   }
   __syncwarp();
@@ -803,7 +803,8 @@ __global__ void k_init(Batch2D b, int64_t n_lcnt) {
   if (i < b.n_table_words) b.table_dst[i] = b.table_src[i];
   if (i < b.n_in16) b.in_dst[i] = b.host_in[i];
   if (i < n_lcnt) b.lcnt[i] = 0;
-  if (i < (int64_t)b.n_chunks * (kChunkWords / 4)) reinterpret_cast<uint4*>(b.seed_bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (b.seed_bits && i < (int64_t)b.n_chunks * (kChunkWords / 4))
+    reinterpret_cast<uint4*>(b.seed_bits)[i] = make_uint4(0u, 0u, 0u, 0u);
   if (b.use_order && i < 2 * kSizeBuckets) b.size_hist[i] = 0;
   if (i < kFlagCount && i != kFlagError) b.flags[i] = i == kFlagGrouped ? 1 : 0;
   if (i == kFlagError && b.clear_error) b.flags[kFlagError] = 0;
@@ -1235,8 +1236,27 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_layers(Batch2D b, Params2D P,
     }
   }
 }
+// The seeds of a lane's 128 points of event e's chunk c, four words: of the
+// chunk's bits (kBits), or, where the run has no memory for those, built from its
+// flags.  (One kernel that asks which: a toy event 33.3 -> 34.0 us.)
+template <bool kBits>
+__device__ __forceinline__ uint4 seed_words(const Batch2D& b, int e, int c) {
+  const int lane = lane_id();
+  if constexpr (kBits) return reinterpret_cast<const uint4*>(b.seed_bits + (int64_t)c * kChunkWords)[lane];
+  const int64_t i0 = b.offsets[e] + (int64_t)(c - b.chunk_start[e]) * kChunk, i1 = b.offsets[e + 1];
+  unsigned w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 4
+  for (int k = 0; k < kChunkWords; ++k) {
+    const int64_t i = i0 + 32 * k + lane;
+    const unsigned v = __ballot_sync(0xffffffffu, i < i1 && b.seed[i] == 1);
+    if (lane == k >> 2) w[k & 3] = v;
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // One block per event: exclusive scan of its chunks' seed counts, which are
 // counted from the bits by a warp per chunk.
+template <bool kBits>
 __global__ void __launch_bounds__(256) k_seed_chunk_scan(Batch2D b) {
   __shared__ int s_n[256];
   __shared__ int s_ws[33];
@@ -1247,7 +1267,7 @@ __global__ void __launch_bounds__(256) k_seed_chunk_scan(Batch2D b) {
   for (int base = c0; base < c1; base += 256) {
 #pragma unroll 4
     for (int k = warp_id(); k < min(256, c1 - base); k += 8) {
-      const uint4 w = reinterpret_cast<const uint4*>(b.seed_bits + (int64_t)(base + k) * kChunkWords)[lane_id()];
+      const uint4 w = seed_words<kBits>(b, e, base + k);
       const int n = (int)__reduce_add_sync(0xffffffffu, (unsigned)(__popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w)));
       if (lane_id() == 0) s_n[k] = n;
     }
@@ -1264,12 +1284,13 @@ __global__ void __launch_bounds__(256) k_seed_chunk_scan(Batch2D b) {
 // Cluster id of each seed = its rank among the event's seeds in index order.
 // One warp per chunk, from the seeds' bits (512 bytes of a chunk; reading its
 // 16 KB of seed flags took 0.325 ms on the 4096-event batch, this 0.121 ms).
+template <bool kBits>
 __global__ void __launch_bounds__(256) k_seed_rank(Batch2D b) {
   pdl_begin();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= b.n_chunks) return;
   const int lane = lane_id();
-  const uint4 w4 = reinterpret_cast<const uint4*>(b.seed_bits + (int64_t)c * kChunkWords)[lane];
+  const uint4 w4 = seed_words<kBits>(b, kBits ? 0 : event_of_chunk(b, c), c);
   const unsigned w[4] = {w4.x, w4.y, w4.z, w4.w};
   const int n = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
   int x = n;
@@ -1400,8 +1421,10 @@ cudaError_t prepare_clue2d_kernels(int device) {
   const void* rest[] = {reinterpret_cast<const void*>(k_init), reinterpret_cast<const void*>(k_count),
                         reinterpret_cast<const void*>(k_layer_scan), reinterpret_cast<const void*>(k_order),
                         reinterpret_cast<const void*>(k_scatter<1>), reinterpret_cast<const void*>(k_scatter<4>),
-                        reinterpret_cast<const void*>(k_seed_chunk_scan),
-                        reinterpret_cast<const void*>(k_seed_rank), reinterpret_cast<const void*>(k_label<false>),
+                        reinterpret_cast<const void*>(k_seed_chunk_scan<true>),
+                        reinterpret_cast<const void*>(k_seed_chunk_scan<false>),
+                        reinterpret_cast<const void*>(k_seed_rank<true>),
+                        reinterpret_cast<const void*>(k_seed_rank<false>), reinterpret_cast<const void*>(k_label<false>),
                         reinterpret_cast<const void*>(k_label<true>)};
   if ((e = cudaFuncSetAttribute(k_scatter<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScatterSmem<1>)) !=
       cudaSuccess)
@@ -1609,18 +1632,19 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
   mark(4);
   {
     NvtxRange r("clue2d/seed_chunk_scan");
+    auto* k = b.seed_bits ? k_seed_chunk_scan<true> : k_seed_chunk_scan<false>;
     if (two_class && b.use_order) {  // behind the join of the two passes
-      k_seed_chunk_scan<<<b.n_events, 256, 0, s>>>(b);
+      k<<<b.n_events, 256, 0, s>>>(b);
       err = cudaGetLastError();
     } else {
-      err = launch_pdl(k_seed_chunk_scan, b.n_events, 256, 0, s, b);
+      err = launch_pdl(k, b.n_events, 256, 0, s, b);
     }
     if (err != cudaSuccess) return err;
   }
   mark(5);
   {
     NvtxRange r("clue2d/seed_rank");
-    if ((err = launch_pdl(k_seed_rank, (nc + 7) / 8, 256, 0, s, b)) != cudaSuccess) return err;
+    if ((err = launch_pdl(b.seed_bits ? k_seed_rank<true> : k_seed_rank<false>, (nc + 7) / 8, 256, 0, s, b)) != cudaSuccess) return err;
   }
   mark(6);
   {

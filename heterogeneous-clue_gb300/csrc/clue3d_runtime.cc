@@ -125,7 +125,7 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
       need[T_IN] = 32 * (size_t)N;
       need[T_OUT] = 28 * (size_t)N;
     }
-    rc = h->arena3d.reserve(need, h->budget > h->arena.total() ? h->budget - h->arena.total() : 0);
+    rc = h->reserve_beside(h->arena3d, need, {&h->arena});
     if (rc) return rc;
     rc = h->stage.reserve(table_bytes);
     if (rc) return rc;

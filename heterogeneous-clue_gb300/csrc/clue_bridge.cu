@@ -441,11 +441,6 @@ int grid_for(int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16));
 }
 
-size_t bridge_budget(const Handle* h) {
-  const size_t used = h->arena.total() + h->arena3d.total();
-  return h->budget > used ? h->budget - used : 0;
-}
-
 }  // namespace
 }  // namespace clue
 
@@ -474,7 +469,7 @@ int clue_bridge_count(clue_handle* hh, int32_t E, const int64_t* off, const int3
     const size_t table_bytes = 8 * (size_t)(E + 1) + 4 * (size_t)nch;
     need[clue::B_TABLES] = table_bytes;
     need[clue::B_COUNT] = 4 * (size_t)E;
-    if ((rc = h->arena_bridge.reserve(need, clue::bridge_budget(h)))) return rc;
+    if ((rc = h->reserve_beside(h->arena_bridge, need, {&h->arena, &h->arena3d}))) return rc;
     if ((rc = h->stage.reserve(table_bytes))) return rc;
     if ((rc = h->nt_host.reserve(4 * (size_t)E))) return rc;
     auto P = [&](int s) { return h->arena_bridge.ptr(s); };
@@ -529,7 +524,7 @@ int clue_bridge_build(clue_handle* hh, const clue_bridge_params* p, int32_t E, c
     need[clue::B_TABLES] = table_bytes;
     need[clue::B_COUNT] = 4 * (size_t)E;
     need[clue::B_SUMS] = sum_bytes;
-    if ((rc = h->arena_bridge.reserve(need, clue::bridge_budget(h)))) return rc;
+    if ((rc = h->reserve_beside(h->arena_bridge, need, {&h->arena, &h->arena3d}))) return rc;
     if ((rc = h->stage.reserve(table_bytes))) return rc;
     if ((rc = h->flags_host.reserve(4 * clue::kFlagCount))) return rc;
     auto P = [&](int s) { return h->arena_bridge.ptr(s); };

@@ -118,7 +118,7 @@ struct Batch2D {
   int32_t* gid = nullptr;
   float* sp[8] = {};          // [N] each: HBM home of layers larger than layer_capacity
   int32_t* sp_tbl = nullptr;  // [grid * kTableInts]
-  uint32_t* seed_bits = nullptr;   // [n_chunks * kChunkWords] the seeds of each chunk
+  uint32_t* seed_bits = nullptr;   // [n_chunks * kChunkWords] the seeds of each chunk (nullptr: ranked from `seed`)
   int32_t* chunk_base = nullptr;   // [n_chunks]
   int32_t* flags = nullptr;        // [kFlagCount]
 };

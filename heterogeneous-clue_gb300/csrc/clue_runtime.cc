@@ -105,6 +105,15 @@ size_t DeviceArena::bytes_after(const std::vector<size_t>& need) const {
   return t;
 }
 
+bool DeviceArena::give_back(int slot) {
+  if (!ptr(slot)) return false;
+  cudaFree(bufs_[slot].p);
+  total_ -= bufs_[slot].bytes;
+  bufs_[slot] = Buf{};
+  ++gen_;
+  return true;
+}
+
 PinnedBuf::~PinnedBuf() {
   if (p) cudaFreeHost(p);
 }
@@ -166,6 +175,18 @@ std::vector<size_t> sizes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bo
   return s;
 }
 
+// Buffers for a run's `need`.  The seed bits (512 bytes per chunk) are worth their
+// room but a run can do without them (its seeds are then ranked from the isSeed
+// flags, 0.325 against 0.121 ms on the 4096-event batch), so they are no reason
+// to refuse one.
+int reserve_run(DeviceArena& a, std::vector<size_t> need, size_t budget) {
+  int rc = a.reserve(need, budget);
+  if (rc != CLUE_ENOMEM) return rc;
+  need[S_CSEED] = 0;
+  a.give_back(S_CSEED);
+  return a.reserve(need, budget);
+}
+
 bool is_pinned_or_device(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -189,8 +210,9 @@ bool host_accessible(const void* const* p, int n) {
   return true;
 }
 
-size_t required_bytes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bool host_io) {
+size_t required_bytes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bool host_io, bool seed_bits) {
   auto s = sizes_2d(E, N, nchunks, grid, host_io);
+  if (!seed_bits) s[S_CSEED] = 0;
   size_t t = 0;
   for (size_t v : s) t += (v + 255) & ~size_t(255);
   return t;
@@ -199,7 +221,7 @@ size_t required_bytes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bool h
 int reserve_2d(Handle* h, int32_t E, int64_t N, bool host_io) {
   const int64_t nchunks = N / kChunk + E;
   const int grid = layer_grid_max(h->tuning, std::max(1, E * kLayers));
-  int rc = h->arena.reserve(sizes_2d(E, N, nchunks, grid, host_io), h->budget);
+  int rc = reserve_run(h->arena, sizes_2d(E, N, nchunks, grid, host_io), h->budget);
   if (!rc) rc = h->stage.reserve(24 * (size_t)(E + 1) + 4 * (size_t)nchunks);
   if (!rc) rc = h->flags_host.reserve(4 * kFlagCount);
   return rc;
@@ -207,7 +229,31 @@ int reserve_2d(Handle* h, int32_t E, int64_t N, bool host_io) {
 
 size_t arena_bytes_after_2d(const Handle* h, int32_t E, int64_t N, int64_t nchunks, bool host_io) {
   const int grid = layer_grid_max(h->tuning, std::max(1, E * kLayers));
-  return h->arena.bytes_after(sizes_2d(E, N, nchunks, grid, host_io));
+  auto need = sizes_2d(E, N, nchunks, grid, host_io);
+  need[S_CSEED] = 0;
+  return h->arena.bytes_after(need) - h->arena.bytes(S_CSEED);
+}
+
+size_t seed_bits_bytes(const Handle* h) { return h->arena.bytes(S_CSEED); }
+
+// Gives back the seed bits of the 2D arenas (no run may be pending).
+bool Handle::give_back_seed_bits() {
+  bool any = arena.give_back(S_CSEED);
+  for (auto& a : arena_pipe) any |= a.give_back(S_CSEED);
+  return any;
+}
+
+// Buffers in `a`, within what the handle's other arenas leave of its budget.
+int Handle::reserve_beside(DeviceArena& a, const std::vector<size_t>& need,
+                           std::initializer_list<const DeviceArena*> others) {
+  auto room = [&] {
+    size_t used = 0;
+    for (const DeviceArena* o : others) used += o->total();
+    return budget > used ? budget - used : 0;
+  };
+  int rc = a.reserve(need, room());
+  if (rc == CLUE_ENOMEM && give_back_seed_bits()) rc = a.reserve(need, room());
+  return rc;
 }
 
 Handle::~Handle() {
@@ -437,7 +483,7 @@ int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nul
   }
   const int64_t nchunks = n_chunks_of(r.E, r.off);
   const int grid = layer_grid_max(h->tuning, std::max(1, r.E * kLayers));
-  rc = h->arena.reserve(sizes_2d(r.E, r.N, nchunks, grid, host_io), h->budget);
+  rc = reserve_run(h->arena, sizes_2d(r.E, r.N, nchunks, grid, host_io), h->budget);
   if (rc) return rc;
   // offsets + chunk table through pinned staging (graph nodes copy from it)
   rc = h->stage.reserve(12 * (size_t)(r.E + 1) + 4 * (size_t)nchunks);
@@ -563,7 +609,7 @@ int run_2d_plain(Handle* h, const Run2D& r) {
     need[S_OUT] = 20 * (size_t)maxn;
   }
   need[S_TABLES] = 24 * (size_t)std::max(r.E, 1);  // the offsets of every event, then their chunk tables
-  rc = h->arena.reserve(need, h->budget);
+  rc = reserve_run(h->arena, need, h->budget);
   if (rc) return rc;
   rc = h->stage.reserve(24 * (size_t)std::max(r.E, 1));
   if (rc) return rc;
@@ -670,32 +716,52 @@ constexpr int kPipePieces = 6;
 int run_2d_pipelined(Handle* h, const Run2D& r) {
   int rc = h->wait_previous();
   if (rc) return rc;
-  // event-aligned cuts
-  const int64_t piece = std::min(kPipePoints, r.N / kPipePieces);
-  std::vector<int32_t> cut{0};
-  for (int32_t e = 0; e < r.E; ++e)
-    if (r.off[e + 1] - r.off[cut.back()] >= piece && e + 1 < r.E) cut.push_back(e + 1);
-  cut.push_back(r.E);
-  const int S = (int)cut.size() - 1;
-  int32_t maxE = 0;
-  int64_t maxN = 0, maxC = 0;
-  for (int i = 0; i < S; ++i) {
-    maxE = std::max(maxE, cut[i + 1] - cut[i]);
-    maxN = std::max(maxN, r.off[cut[i + 1]] - r.off[cut[i]]);
-    maxC = std::max(maxC, n_chunks_of(cut[i + 1] - cut[i], r.off + cut[i]));
-  }
-  const int grid = layer_grid_max(h->tuning, std::max(1, maxE * kLayers));
-  const auto need = sizes_2d(maxE, maxN, maxC, grid, true);
   DeviceArena* slot_arena[kPipeSlots];
   slot_arena[0] = &h->arena;
   for (int k = 1; k < kPipeSlots; ++k) slot_arena[k] = &h->arena_pipe[k - 1];
-  if ((rc = h->arena.reserve(need, h->budget))) return rc;
-  for (int k = 1; k < kPipeSlots; ++k) {
-    size_t used = h->arena3d.total() + h->arena_bridge.total();
-    for (int j = 0; j < kPipeSlots; ++j)
-      if (j != k) used += slot_arena[j]->total();
-    if ((rc = slot_arena[k]->reserve(need, h->budget > used ? h->budget - used : 0))) return rc;
+  std::vector<int32_t> cut;
+  // event-aligned cuts into sub-batches of `piece` points, and the slots' buffers for them
+  auto plan = [&](int64_t piece) {
+    cut.assign(1, 0);
+    for (int32_t e = 0; e < r.E; ++e)
+      if (r.off[e + 1] - r.off[cut.back()] >= piece && e + 1 < r.E) cut.push_back(e + 1);
+    cut.push_back(r.E);
+    int32_t maxE = 0;
+    int64_t maxN = 0, maxC = 0;
+    for (size_t i = 0; i + 1 < cut.size(); ++i) {
+      maxE = std::max(maxE, cut[i + 1] - cut[i]);
+      maxN = std::max(maxN, r.off[cut[i + 1]] - r.off[cut[i]]);
+      maxC = std::max(maxC, n_chunks_of(cut[i + 1] - cut[i], r.off + cut[i]));
+    }
+    const int grid = layer_grid_max(h->tuning, std::max(1, maxE * kLayers));
+    auto need = sizes_2d(maxE, maxN, maxC, grid, true);
+    auto reserve = [&]() {
+      int rc = h->arena.reserve(need, h->budget);
+      for (int k = 1; k < kPipeSlots && !rc; ++k) {
+        size_t used = h->arena3d.total() + h->arena_bridge.total();
+        for (int j = 0; j < kPipeSlots; ++j)
+          if (j != k) used += slot_arena[j]->total();
+        rc = slot_arena[k]->reserve(need, h->budget > used ? h->budget - used : 0);
+      }
+      return rc;
+    };
+    int rc = reserve();
+    if (rc == CLUE_ENOMEM) {  // without the seed bits, see reserve_run
+      need[S_CSEED] = 0;
+      h->give_back_seed_bits();
+      rc = reserve();
+    }
+    return rc;
+  };
+  rc = plan(std::min(kPipePoints, r.N / kPipePieces));
+  if (rc == CLUE_ENOMEM && r.N / kPipePieces < kPipePoints) {
+    // a smaller piece may end on a larger sub-batch, one that holds a large
+    // event: what fits the budget in pieces of kPipePoints is taken
+    for (auto* a : slot_arena) a->release();
+    rc = plan(kPipePoints);
   }
+  if (rc) return rc;
+  const int S = (int)cut.size() - 1;
   // pinned staging: per sub-batch its rebased offsets and chunk table
   std::vector<size_t> st_off(S + 1, 0);
   for (int i = 0; i < S; ++i) {

@@ -5,6 +5,7 @@
 
 #include <cstddef>
 #include <exception>
+#include <initializer_list>
 #include <new>
 #include <cstdint>
 #include <vector>
@@ -41,6 +42,8 @@ class DeviceArena {
   // Device bytes the arena would hold after reserve(need) without the growth
   // margin (the margin is only taken when the budget has room for it).
   size_t bytes_after(const std::vector<size_t>& need) const;
+  bool give_back(int slot);  // frees one buffer; whether there was one
+  size_t bytes(int slot) const { return slot < (int)bufs_.size() ? bufs_[slot].bytes : 0; }
   void* ptr(int slot) const { return slot < (int)bufs_.size() ? bufs_[slot].p : nullptr; }
   size_t total() const { return total_; }
   uint64_t generation() const { return gen_; }  // bumped whenever a buffer is (re)allocated
@@ -88,15 +91,16 @@ struct GraphKey {
   }
 };
 
-size_t required_bytes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bool host_io);
+size_t required_bytes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bool host_io, bool seed_bits = true);
 struct Handle;
 // Sizes the handle's 2D buffers for a batch of E events and N points ahead of
 // time (a server slot does this at start so that its first batches do not
 // allocate).
 int reserve_2d(Handle* h, int32_t E, int64_t N, bool host_io);
-// Device bytes the handle's 2D arena would hold after sizing it for a batch of
-// E events, N points and nchunks chunks (the batch's own chunk count).
+// Device bytes that the handle's 2D arena would hold at least after sizing it for
+// a batch of E events, N points and nchunks chunks (the batch's own chunk count).
 size_t arena_bytes_after_2d(const Handle* h, int32_t E, int64_t N, int64_t nchunks, bool host_io);
+size_t seed_bits_bytes(const Handle* h);  // of those it holds now
 
 // Internal run flag: host (pinned) buffers, but return once the work is
 // queued; completion is seen through Handle::done_event.  Used by the server.
@@ -148,6 +152,8 @@ struct Handle {
 
   ~Handle();
   int wait_previous();
+  bool give_back_seed_bits();
+  int reserve_beside(DeviceArena& a, const std::vector<size_t>& need, std::initializer_list<const DeviceArena*> others);
   int wait_queued();
   int ensure_side(int n_events);
   const SideStream* side_stream() const { return side.stream && side.join ? &side : nullptr; }

@@ -64,7 +64,7 @@ struct Slot {
   bool busy = false;      // requests taken (staging, on the device or delivering results)
   bool launched = false;  // the batch is queued on the device
   int64_t batch_points = 0;  // batches are cut at this size: the buffers sized at start
-  size_t base_bytes = 0;     // device bytes of those start-up buffers
+  size_t base_bytes = 0;     // device bytes of those start-up buffers, without the seed bits
 };
 
 class Server {
@@ -91,7 +91,7 @@ class Server {
       while (hi - lo > 1) {
         const int64_t mid = (lo + hi) / 2;
         const int64_t chunks = mid / kChunk + cfg_.max_batch_events;
-        if (required_bytes_2d(cfg_.max_batch_events, mid, chunks, grid, true) <= base_share) lo = mid; else hi = mid;
+        if (required_bytes_2d(cfg_.max_batch_events, mid, chunks, grid, true, false) <= base_share) lo = mid; else hi = mid;
       }
       if (lo < 1) return set_error(CLUE_ENOMEM, "budget too small for one in-flight batch");
       // resident buffers for batches up to 8M points, so that ordinary loads
@@ -102,7 +102,7 @@ class Server {
       if (!rc) rc = s.in.reserve(16 * (size_t)s.batch_points);
       if (!rc) rc = s.out.reserve(20 * (size_t)s.batch_points);
       if (rc) return rc;
-      s.base_bytes = hh->arena.total();
+      s.base_bytes = hh->arena.total() - seed_bits_bytes(hh);
     }
     // the largest single event ever admitted: it fits the budget while every
     // other slot holds only its start-up buffers
@@ -360,9 +360,11 @@ class Server {
       for (auto& o : slots_) {
         Handle* ho = reinterpret_cast<Handle*>(o.h);
         if (&o == &s || o.busy || ho->arena.total() <= o.base_bytes) continue;
+        if (ho->give_back_seed_bits() && ho->arena.total() <= o.base_bytes) continue;
         ho->arena.release();
         ho->budget = budget_;
         reserve_2d(ho, cfg_.max_batch_events, o.batch_points, true);
+        ho->give_back_seed_bits();
         o.base_bytes = ho->arena.total();
       }
       g.lock();
