@@ -316,7 +316,9 @@ struct RowsGlobal {
 // an HGCAL event: a good half lies below eta 1.5, in the first eta row, so that
 // row holds some thirty entries and often three in a column; 1.24M such clusters
 // of 200 events: columns counted from global memory 0.67 ms, from the bytes by a
-// binary search 0.43.)
+// binary search 0.43.  Both ends of a window are searched for: with the entries
+// counted on from its first one, 20,000 clusters on a line of phi, some hundred to
+// a column, took 1.23 ms, 0.65 now.)
 constexpr int kRowStartBits = 12, kRowSlotBits = 8;
 constexpr int kRowRepeat = 1 << 30;  // a column holds two entries
 constexpr int kRowWalk = 1 << 29;    // counted by its entries' columns
@@ -580,12 +582,8 @@ __device__ __forceinline__ RowRuns row_runs(const RowsStaged& v, int r, const Ph
       const uint8_t* cs = v.cols + 4 * ((rs >> kRowStartBits) & ((1 << kRowSlotBits) - 1)) - o.s;
       auto col = [&](int q) { return (rs & kRowCols) ? (int)cs[q] : v.col(q); };
       o.qa = first_at(o.s, t, a0, col);
-      int q = o.qa;
-      while (q < t && col(q) < a1) ++q;
-      o.na = q - o.qa;
-      q = o.s;
-      while (q < t && col(q) < a1 - kPhiBins) ++q;
-      o.nb = q - o.s;
+      o.na = first_at(o.qa, t, a1, col) - o.qa;
+      o.nb = f.wraps() ? first_at(o.s, o.qa, a1 - kPhiBins, col) - o.s : 0;
     } else {
       const uint32_t* p = v.rep + 4 * ((rs >> kRowStartBits) & ((1 << kRowSlotBits) - 1));
       o.na += __popc(f.arc_a(p));
