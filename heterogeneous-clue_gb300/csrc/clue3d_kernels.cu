@@ -690,8 +690,13 @@ static_assert(kSlabMaxCand < 1 << kRowStartBits && kSlabSlots <= 1 << kRowSlotBi
 constexpr size_t kSlabSmem = 16 * (size_t)kSlabMaxCand + 16 * (size_t)kSlabMaxRows + 16 * (size_t)kSlabSlots +
                              8 * (size_t)(kSlabMaxRows + 1) + 4 * (size_t)kSlabColWords;
 
-template <bool kDensity, bool kParts>
+// How a launch takes its slabs: each in one part, or in halves or single layers
+// where its staging does not fit, or all from global memory (see launch_clue3d).
+enum SlabMode { kWhole, kInParts, kGlobal };
+
+template <bool kDensity, SlabMode kMode>
 __global__ void __launch_bounds__(kSlabThreads, 5) k3_search(Batch3D b, Params3D P, int n_slabs) {
+  constexpr bool kParts = kMode == kInParts;
   extern __shared__ __align__(16) unsigned char sm3[];
   float4* s_cand = reinterpret_cast<float4*>(sm3);
   uint32_t* s_mask = reinterpret_cast<uint32_t*>(s_cand + kSlabMaxCand);
@@ -714,8 +719,6 @@ __global__ void __launch_bounds__(kSlabThreads, 5) k3_search(Batch3D b, Params3D
   // phi bin 126 in its last eta row
   auto layers_end = [&](int l) { return rs[l * kEtaBins + (l == P.n_layers ? 1 : 0)]; };
   if (rs[L0 * kEtaBins] >= layers_end(L1)) return;
-  // kParts: the slab in one part, or in halves or single layers where its staging
-  // does not fit (see launch_clue3d)
   for (int La = L0, Lb; La < L1; La = kParts ? Lb : L1) {
     // rows of layers [La - sib, Lb + sib) and the first row after them (the
     // reference's eta window reaches row 34 of a layer, the next layer's row 0)
@@ -727,7 +730,7 @@ __global__ void __launch_bounds__(kSlabThreads, 5) k3_search(Batch3D b, Params3D
       nrows = row_hi - row_lo + 1;
       pos_lo = rs[row_lo];
       pos_hi = rs[row_hi + 1];
-      staged = nrows <= kSlabMaxRows && pos_hi - pos_lo <= kSlabMaxCand;
+      staged = kMode != kGlobal && nrows <= kSlabMaxRows && pos_hi - pos_lo <= kSlabMaxCand;
       if (staged || !kParts) break;
       if (Lb - La == 1) {  // not even one layer's: from global memory, together
         Lb = L1;
@@ -963,7 +966,8 @@ __global__ void k3_label(Batch3D b) {
 
 cudaError_t prepare_clue3d_kernels() {
   // more than the 48 KB a kernel may use without asking
-  for (auto* k : {k3_search<true, false>, k3_search<true, true>, k3_search<false, false>, k3_search<false, true>}) {
+  for (auto* k : {k3_search<true, kWhole>, k3_search<true, kInParts>, k3_search<true, kGlobal>, k3_search<false, kWhole>,
+                  k3_search<false, kInParts>, k3_search<false, kGlobal>}) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem);
     if (e != cudaSuccess) return e;
   }
@@ -1000,28 +1004,36 @@ cudaError_t launch_clue3d(const Batch3D& b, const Params3D& p, cudaStream_t s) {
   const int n_slabs = (p.n_layers + kSlabLayers - 1) / kSlabLayers;
   const int64_t slab_blocks = (int64_t)b.n_events * n_slabs;
   if (slab_blocks > INT32_MAX) return cudaErrorInvalidValue;
-  // Whether the batch's largest event, its clusters spread evenly over the
-  // layers, would fill seven eighths of the staging area (1,792 candidates to a
-  // slab: six standard deviations below its 2,048): such slabs may have to be
-  // searched in parts (100 events of 20,000 clusters with three sibling layers,
-  // 2,130 candidates to a slab: 1.42 ms from global memory, 0.59 in two parts).
+  // Slabs may have to be searched in parts where the batch's largest event, its
+  // clusters spread evenly over the layers, would fill seven eighths of the
+  // staging area (1,792 candidates to a slab: six standard deviations below its
+  // 2,048; 100 events of 20,000 clusters with three sibling layers, 2,130
+  // candidates to a slab: 1.42 ms from global memory, 0.59 in two parts).
   // Other batches keep the form without the loop (1,000 events of up to 20,000 with
   // two: 2.07 ms, 2.10 with it); a slab that is crowded all the same then reads
-  // global memory.
-  auto parts = [&](int sib) {
-    return (int64_t)b.max_event * (kSlabLayers + 2 * (int64_t)std::clamp(sib, 0, p.n_layers)) >
-           (int64_t)p.n_layers * (kSlabMaxCand / 8 * 7);
+  // global memory.  Where the rows of a slab exceed the area (four sibling layers
+  // and more) none is staged, and the memory is left to the L1 cache (50
+  // events of 10,000 with six: 0.577 ms beside an unused area, 0.466; with four:
+  // 0.366 in halves, 0.351, and with half the clusters in one eta row 0.454 and
+  // 0.356; with five, which takes single layers, 0.650 and 0.408).
+  auto mode = [&](int sib) {
+    const int64_t window = kSlabLayers + 2 * (int64_t)std::clamp(sib, 0, p.n_layers);
+    if (std::min<int64_t>(window, p.n_layers) * kEtaBins + 1 > kSlabMaxRows) return kGlobal;
+    return b.max_event * window > (int64_t)p.n_layers * (kSlabMaxCand / 8 * 7) ? kInParts : kWhole;
+  };
+  auto search = [&](auto* whole, auto* parts, auto* global, int sib) {
+    const SlabMode m = mode(sib);
+    return launch_pdl(m == kWhole ? whole : m == kInParts ? parts : global, (unsigned)slab_blocks, kSlabThreads,
+                      m == kGlobal ? 0 : kSlabSmem, s, b, p, n_slabs);
   };
   {
     NvtxRange r("clue3d/density");
-    err = launch_pdl(parts(p.dens_sib) ? k3_search<true, true> : k3_search<true, false>, (unsigned)slab_blocks, kSlabThreads,
-                     kSlabSmem, s, b, p, n_slabs);
+    err = search(k3_search<true, kWhole>, k3_search<true, kInParts>, k3_search<true, kGlobal>, p.dens_sib);
     if (err != cudaSuccess) return err;
   }
   {
     NvtxRange r("clue3d/nearest_higher");
-    err = launch_pdl(parts(p.nh_sib) ? k3_search<false, true> : k3_search<false, false>, (unsigned)slab_blocks, kSlabThreads,
-                     kSlabSmem, s, b, p, n_slabs);
+    err = search(k3_search<false, kWhole>, k3_search<false, kInParts>, k3_search<false, kGlobal>, p.nh_sib);
     if (err != cudaSuccess) return err;
   }
   {
