@@ -7,6 +7,7 @@
 // PointsCloudCUDA per event from the caching allocator; here a handle owns
 // grow-only device buffers sized for the largest batch seen, capped by a
 // budget, and nothing is allocated on the steady-state path.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -187,6 +188,40 @@ int reserve_run(DeviceArena& a, std::vector<size_t> need, size_t budget) {
   return a.reserve(need, budget);
 }
 
+// Whether host arrays of `bytes` each move in one copy: they lie back to back, in
+// one block of page-locked memory or all in pageable memory.  (A copy that runs
+// from one page-locked block into the next, where two lie back to back, is an
+// invalid value to the driver.)
+bool one_copy(std::initializer_list<const void*> arrays, size_t bytes) {
+  const char* first = static_cast<const char*>(*arrays.begin());
+  size_t k = 0;
+  for (const void* a : arrays)
+    if (a != first + bytes * k++) return false;
+  const void* ends[2] = {first, first + bytes * (k - 1)};
+  bool pageable = true;
+  for (const void* a : ends) {
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, a) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    pageable &= attr.type == cudaMemoryTypeUnregistered;
+  }
+  if (pageable) return true;
+  static const auto get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found{};
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found) != cudaSuccess)
+      cudaGetLastError();
+    return reinterpret_cast<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>(f);
+  }();
+  const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(first);
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  return get && get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) == CUDA_SUCCESS &&
+         get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) == CUDA_SUCCESS && p >= start && p - start + bytes * k <= size;
+}
+
 bool is_pinned_or_device(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -360,11 +395,13 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
   cudaStream_t s = h->stream;
   cudaError_t e;
   const size_t n4 = 4 * (size_t)r.N;
-  if (host_io && !b.host_in) {
-    // back-to-back host arrays (a server's staging) move in one copy
-    const char* hx = reinterpret_cast<const char*>(r.x);
-    if (reinterpret_cast<const char*>(r.y) == hx + n4 && reinterpret_cast<const char*>(r.layer) == hx + 2 * n4 &&
-        reinterpret_cast<const char*>(r.w) == hx + 3 * n4) {
+  // back-to-back host arrays (a server's staging is laid out so) move in one copy
+  const bool known = r.flags & kAsyncHostIO, copies = host_io && !b.host_in;
+  const bool in_one = known || (copies && one_copy({r.x, r.y, r.layer, r.w}, n4));
+  const bool out_one = known || (copies && one_copy({r.out->rho, r.out->delta, r.out->nearestHigher, r.out->isSeed,
+                                                     r.out->clusterIndex}, n4));
+  if (copies) {
+    if (in_one) {
       if ((e = cudaMemcpyAsync((void*)b.x, r.x, 4 * n4, cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return cuda_error(e, "H2D points");
     } else if ((e = cudaMemcpyAsync((void*)b.x, r.x, n4, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
@@ -378,11 +415,7 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
   if (e != cudaSuccess) return cuda_error(e, "launching CLUE kernels");
   if (host_io && !b.host_out) {
     const clue_outputs* o = r.out;
-    const char* ho = reinterpret_cast<const char*>(o->rho);
-    if (reinterpret_cast<const char*>(o->delta) == ho + n4 &&
-        reinterpret_cast<const char*>(o->nearestHigher) == ho + 2 * n4 &&
-        reinterpret_cast<const char*>(o->isSeed) == ho + 3 * n4 &&
-        reinterpret_cast<const char*>(o->clusterIndex) == ho + 4 * n4) {
+    if (out_one) {
       if ((e = cudaMemcpyAsync(o->rho, b.rho, 5 * n4, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return cuda_error(e, "D2H outputs");
     } else if ((e = cudaMemcpyAsync(o->rho, b.rho, n4, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
