@@ -1,6 +1,7 @@
 // Host side of CLUE3D: parameters, buffers and the clue3d_* C entry points.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -133,7 +134,9 @@ int clue3d_run_batch(clue_handle* hh, const clue3d_params* prm, int32_t E, const
     if (rc) return rc;
     rc = h->nt_host.reserve(4 * (size_t)E);
     if (rc) return rc;
-    const bool staged = host_io && N <= kStagedIoPoints && host_accessible(ins, 8) && host_accessible(outs, 7);
+    const void* io[15];
+    std::copy_n(outs, 7, std::copy_n(ins, 8, io));
+    const bool staged = host_io && stages_io(io, 15, N);
     if (staged) {
       if ((rc = h->io_stage.reserve(60 * (size_t)N)) || (rc = h->wait_queued())) return rc;
     }

@@ -233,16 +233,19 @@ bool is_pinned_or_device(const void* p) {
 
 }  // namespace
 
-bool host_accessible(const void* const* p, int n) {
+bool stages_io(const void* const* p, int n, int64_t N) {
+  if (N > kStagedIoPoints) return false;
+  bool pageable = false;
   for (int i = 0; i < n; ++i) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p[i]) != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
-    if (a.type == cudaMemoryTypeDevice) return false;
+    if (a.type == cudaMemoryTypeDevice) return false;  // not for the CPU to read or write
+    pageable |= a.type == cudaMemoryTypeUnregistered;
   }
-  return true;
+  return pageable || 4 * n * N <= kStagedIoPinnedBytes;
 }
 
 size_t required_bytes_2d(int32_t E, int64_t N, int64_t nchunks, int grid, bool host_io, bool seed_bits) {
@@ -498,7 +501,7 @@ int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nul
   // a small host run: through page-locked staging, inputs back to back, then outputs
   const void* io[9] = {r.x, r.y, r.layer, r.w, r.out->rho, r.out->delta, r.out->nearestHigher, r.out->isSeed,
                        r.out->clusterIndex};
-  const bool staged = host_io && !(r.flags & kAsyncHostIO) && r.N <= kStagedIoPoints && host_accessible(io, 9);
+  const bool staged = host_io && !(r.flags & kAsyncHostIO) && stages_io(io, 9, r.N);
   clue_outputs staged_out;
   if (staged) {
     const size_t n4 = 4 * (size_t)r.N;

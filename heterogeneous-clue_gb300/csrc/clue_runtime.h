@@ -109,14 +109,18 @@ constexpr int kAsyncHostIO = 0x100;
 // Host-memory runs of up to this many points (or layer clusters) go through
 // page-locked staging that the first kernel reads and the last one writes: two
 // host copies instead of a stream copy per array (9 or 15 of them, each
-// staged by the driver).  Producer call on 5k / 25k points 105 -> 64 / 143 ->
-// 105 us; at 50k points the host copies cost more (152 -> 163 us).  CLUE3D on
-// 5k layer clusters 168 -> 118 us, on 50k 252 -> 300 us.  The calling thread
-// reads the arrays, so on a caller's stream it first waits for the work queued
-// there, which may fill them (Handle::wait_queued).
+// staged by the driver).  Producer call on 5k / 25k points 103 -> 52 / 136 ->
+// 92 us; at 50k points the host copies cost more (152 -> 163 us).  CLUE3D on
+// 5k / 20k layer clusters 158 -> 97 / 302 -> 230 us, on 50k 252 -> 300 us.  The
+// calling thread reads the arrays, so on a caller's stream it first waits for the
+// work queued there, which may fill them (Handle::wait_queued).
 constexpr int64_t kStagedIoPoints = int64_t(32) << 10;
-// Whether the CPU may read and write all of these arrays.
-bool host_accessible(const void* const* p, int n);
+// Page-locked arrays need no staging by the driver, so for them fewer bytes pay:
+// 8k / 12k / 16k points 69-74 -> 57-64 / 70-74 -> 66-72 / 70-75 -> 74-80 us (by
+// direct launches and replayed), CLUE3D on 5k / 10k 115 -> 99 / 128 -> 133 us.
+constexpr int64_t kStagedIoPinnedBytes = int64_t(448) << 10;
+// Whether a host-memory run of N points with these n arrays goes that way.
+bool stages_io(const void* const* p, int n, int64_t N);
 
 // Device slots of the pipelined host-memory path (sub-batches in flight).
 constexpr int kPipeSlots = 2;
