@@ -381,6 +381,15 @@ struct Run2D {
   int flags;
 };
 
+// Whether none of a run's arrays is pageable.
+bool pages_locked(const Run2D& r) {
+  for (const void* p : {(const void*)r.x, (const void*)r.y, (const void*)r.layer, (const void*)r.w, (const void*)r.out->rho,
+                        (const void*)r.out->delta, (const void*)r.out->nearestHigher, (const void*)r.out->isSeed,
+                        (const void*)r.out->clusterIndex})
+    if (!is_pinned_or_device(p)) return false;
+  return true;
+}
+
 int validate_offsets(int32_t E, const int64_t* off) {
   if (E < 0) return set_error(CLUE_EINVAL, "n_events < 0");
   if (E == 0) return CLUE_OK;
@@ -550,10 +559,7 @@ int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nul
   bool use_graph = !(r.flags & CLUE_NO_GRAPH) && !stage_events;
   if (use_graph && host_io && !staged) {
     // graph memcpy nodes need page-locked host memory
-    use_graph = is_pinned_or_device(r.x) && is_pinned_or_device(r.y) && is_pinned_or_device(r.layer) &&
-                is_pinned_or_device(r.w) && is_pinned_or_device(r.out->rho) &&
-                is_pinned_or_device(r.out->delta) && is_pinned_or_device(r.out->nearestHigher) &&
-                is_pinned_or_device(r.out->isSeed) && is_pinned_or_device(r.out->clusterIndex);
+    use_graph = pages_locked(r);
   }
   cudaError_t e;
   int64_t kernels = 0;
@@ -745,9 +751,12 @@ int run_2d_plain(Handle* h, const Run2D& r) {
 // copy into the first and out of the last overlap nothing, which with four
 // pieces of 8M points was a third of the time.  512 events (27.5M points):
 // 4.93 ms in pieces of 8M, 4.65 of 4M, 4.52 of 3M, 4.59 of 2M; 108M points
-// and more are cut as before.
+// and more are cut as before.  Pageable arrays pass through the driver's own
+// staging, whose start each copy pays, and overlap little: a third there (18M
+// points: 4.88 ms in pieces of 8M, 5.08 in sixths, 4.71 in thirds; 35M: 9.13,
+// 9.00, 8.81).
 constexpr int64_t kPipePoints = int64_t(8) << 20;
-constexpr int kPipePieces = 6;
+constexpr int kPipePieces = 6, kPipePiecesPageable = 3;
 
 int run_2d_pipelined(Handle* h, const Run2D& r) {
   int rc = h->wait_previous();
@@ -789,12 +798,17 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
     }
     return rc;
   };
-  rc = plan(std::min(kPipePoints, r.N / kPipePieces));
-  if (rc == CLUE_ENOMEM && r.N / kPipePieces < kPipePoints) {
-    // a smaller piece may end on a larger sub-batch, one that holds a large
-    // event: what fits the budget in pieces of kPipePoints is taken
-    for (auto* a : slot_arena) a->release();
-    rc = plan(kPipePoints);
+  // What the budget takes in smaller pieces, or in pieces of kPipePoints, is taken
+  // (smaller ones may end on a larger sub-batch, one that holds a large event).
+  const int64_t pieces[3] = {r.N / (pages_locked(r) ? kPipePieces : kPipePiecesPageable), r.N / kPipePieces, kPipePoints};
+  int64_t piece = 0;
+  rc = CLUE_ENOMEM;
+  for (int i = 0; i < 3 && rc == CLUE_ENOMEM; ++i) {
+    if (i && std::min(kPipePoints, pieces[i]) == piece) continue;
+    piece = std::min(kPipePoints, pieces[i]);
+    if (i)
+      for (auto* a : slot_arena) a->release();
+    rc = plan(piece);
   }
   if (rc) return rc;
   const int S = (int)cut.size() - 1;

@@ -139,10 +139,12 @@ def test_beside_clue3d_and_the_bridge(cuda_lib):
 
 
 @pytest.mark.parametrize("sizes,slot", [((9000000, 9000000), (9000000,)),
-                                        ((4000000, 3450000, 1100000, 12000000), (4000000, 3450000, 4550000))])
+                                        ((4000000, 3450000, 1100000, 12000000), (4000000, 3450000, 4550000)),
+                                        ((1000000,) * 24, (1000000,) * 4)])
 def test_pipelined_host_batches(cuda_lib, sizes, slot):
     """Two slots of a sub-batch each; the second case ends on a larger sub-batch
-    in sixths of the batch (1.1 + 12M points) than in pieces of 8M (12M)."""
+    in thirds and sixths of the batch (1.1 + 12M points) than in pieces of 8M (12M),
+    the third has room for sixths only."""
     off, ev = _batch(sizes, 7, False)
     free = C.Clusterizer(*PRM)
     want = free.run_batch(off, *[ev[k] for k in FIELDS])
