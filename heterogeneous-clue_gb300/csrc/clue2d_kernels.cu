@@ -1255,18 +1255,19 @@ __device__ __forceinline__ uint4 seed_words(const Batch2D& b, int e, int c) {
 }
 
 // One block per event: exclusive scan of its chunks' seed counts, which are
-// counted from the bits by a warp per chunk.
-template <bool kBits>
-__global__ void __launch_bounds__(256) k_seed_chunk_scan(Batch2D b) {
-  __shared__ int s_n[256];
+// counted from the bits by a warp per chunk.  The bits of large events come
+// through one SM, so their blocks are as wide as they go (see launch_clue2d).
+template <bool kBits, int NT>
+__global__ void __launch_bounds__(NT) k_seed_chunk_scan(Batch2D b) {
+  __shared__ int s_n[NT];
   __shared__ int s_ws[33];
   pdl_begin();
   const int e = blockIdx.x;
   const int c0 = b.chunk_start[e], c1 = b.chunk_start[e + 1];
   int run = 0;
-  for (int base = c0; base < c1; base += 256) {
+  for (int base = c0; base < c1; base += NT) {
 #pragma unroll 4
-    for (int k = warp_id(); k < min(256, c1 - base); k += 8) {
+    for (int k = warp_id(); k < min(NT, c1 - base); k += NT / 32) {
       const uint4 w = seed_words<kBits>(b, e, base + k);
       const int n = (int)__reduce_add_sync(0xffffffffu, (unsigned)(__popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w)));
       if (lane_id() == 0) s_n[k] = n;
@@ -1275,7 +1276,7 @@ __global__ void __launch_bounds__(256) k_seed_chunk_scan(Batch2D b) {
     const int c = base + threadIdx.x;
     const int v = c < c1 ? s_n[threadIdx.x] : 0;
     int total;
-    const int x = block_inclusive_scan<256>(v, s_ws, &total);
+    const int x = block_inclusive_scan<NT>(v, s_ws, &total);
     if (c < c1) b.chunk_base[c] = run + x - v;
     run += total;
   }
@@ -1421,8 +1422,9 @@ cudaError_t prepare_clue2d_kernels(int device) {
   const void* rest[] = {reinterpret_cast<const void*>(k_init), reinterpret_cast<const void*>(k_count),
                         reinterpret_cast<const void*>(k_layer_scan), reinterpret_cast<const void*>(k_order),
                         reinterpret_cast<const void*>(k_scatter<1>), reinterpret_cast<const void*>(k_scatter<4>),
-                        reinterpret_cast<const void*>(k_seed_chunk_scan<true>),
-                        reinterpret_cast<const void*>(k_seed_chunk_scan<false>),
+                        reinterpret_cast<const void*>(k_seed_chunk_scan<true, 256>),
+                        reinterpret_cast<const void*>(k_seed_chunk_scan<true, 1024>),
+                        reinterpret_cast<const void*>(k_seed_chunk_scan<false, 1024>),
                         reinterpret_cast<const void*>(k_seed_rank<true>),
                         reinterpret_cast<const void*>(k_seed_rank<false>), reinterpret_cast<const void*>(k_label<false>),
                         reinterpret_cast<const void*>(k_label<true>)};
@@ -1632,12 +1634,17 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
   mark(4);
   {
     NvtxRange r("clue2d/seed_chunk_scan");
-    auto* k = b.seed_bits ? k_seed_chunk_scan<true> : k_seed_chunk_scan<false>;
+    // from 24 chunks per event on (100,000 points; fewer are done in the same time
+    // by narrow blocks, which more events share an SM with): one event of 9M points
+    // 109 -> 33 us, 200 of 325,000 10 -> 8
+    const bool wide = !b.seed_bits || nc >= 24 * (int64_t)b.n_events;
+    auto* k = !b.seed_bits ? k_seed_chunk_scan<false, 1024> : wide ? k_seed_chunk_scan<true, 1024> : k_seed_chunk_scan<true, 256>;
+    const int threads = wide ? 1024 : 256;
     if (two_class && b.use_order) {  // behind the join of the two passes
-      k<<<b.n_events, 256, 0, s>>>(b);
+      k<<<b.n_events, threads, 0, s>>>(b);
       err = cudaGetLastError();
     } else {
-      err = launch_pdl(k, b.n_events, 256, 0, s, b);
+      err = launch_pdl(k, b.n_events, threads, 0, s, b);
     }
     if (err != cudaSuccess) return err;
   }
