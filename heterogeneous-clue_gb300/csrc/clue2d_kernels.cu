@@ -1028,12 +1028,16 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
   __shared__ int s_at[kLayers];    // their first slot here
   __shared__ int s_base[kLayers];  // their first position
   __shared__ int s_total;
+  __shared__ int s_it;
   const int lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
   pdl_begin();
   if (b.flags[kFlagGrouped]) return;  // input already grouped by layer
-  for (int it = blockIdx.x; it < b.n_chunks * kSlices; it += gridDim.x) {
+  // a resident block's next slices from a ticket, taken while one is done
+  const bool ticket = b.n_chunks * kSlices > 2 * (int)gridDim.x;
+  for (int it = blockIdx.x; it < b.n_chunks * kSlices;) {
     const int c = it / kSlices;
+    if (ticket && threadIdx.x == kChunkThreads - 1) s_it = (int)gridDim.x + atomicAdd(&b.flags[kFlagTicketScatter], 1);
     for (int l = threadIdx.x; l < kLayers; l += kChunkThreads) s_cnt[l] = 0;
     if (threadIdx.x == 0) s_e = event_of_chunk(b, c);
     __syncthreads();
@@ -1113,6 +1117,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(Batch2D b) {
         b.gid[pos] = (int32_t)r.w;
       }
     }
+    it = ticket ? s_it : it + (int)gridDim.x;
     __syncthreads();  // the shared arrays of the next slice
   }
 }
@@ -1533,16 +1538,14 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
   // stay on chip.  Measured per producer call: 0.177 -> 0.131 ms on events of
   // 150k-200k points, 0.136 -> 0.117 ms on 50k-150k, 0.113 -> 0.101 ms on 5k-20k.
   Tuning2D tt = t;
-  {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (n_items <= sms) {
-      tt.threads = 1024;
-      tt.layer_capacity = std::max(std::max(t.layer_capacity, t.big_capacity), 4096);
-      tt.ctas_per_sm = 0;
-      tt.big_threads = tt.big_capacity = 0;
-    }
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (n_items <= sms) {
+    tt.threads = 1024;
+    tt.layer_capacity = std::max(std::max(t.layer_capacity, t.big_capacity), 4096);
+    tt.ctas_per_sm = 0;
+    tt.big_threads = tt.big_capacity = 0;
   }
   const bool two_class = tt.big_threads > 0 && tt.big_capacity > tt.layer_capacity;
   b.use_order = layers_ordered(t, n_items) ? 1 : 0;
@@ -1585,10 +1588,15 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
   mark(2);
   {
     NvtxRange r("clue2d/scatter");
-    // a resident grid: grouped input has nothing to do here (57 -> 4 us on the
-    // 4096-event batch against a block per chunk)
-    err = nc <= 152 ? launch_pdl(k_scatter<4>, nc * 4, kChunkThreads, kScatterSmem<4>, s, b)
-                    : launch_pdl(k_scatter<1>, std::min(nc, 152 * 3), kChunkThreads, kScatterSmem<1>, s, b);
+    // A resident grid, two blocks of 64 registers a thread per SM: grouped input
+    // has nothing to do here (57 -> 4 us on the 4096-event batch against a block
+    // per chunk), and of three per SM every third block started with as many
+    // chunks to go as the others when those were done (15.3M shuffled points 0.198
+    // -> 0.160 ms, 32.5M 0.407 -> 0.323).  Up to five chunks per SM leave
+    // two and a few threes to a block of two per SM, and take three (2.5M points 244
+    // us in all, 247).
+    err = nc <= sms ? launch_pdl(k_scatter<4>, nc * 4, kChunkThreads, kScatterSmem<4>, s, b)
+                    : launch_pdl(k_scatter<1>, std::min(nc, sms * (nc <= 5 * sms ? 3 : 2)), kChunkThreads, kScatterSmem<1>, s, b);
     if (err != cudaSuccess) return err;
   }
   mark(3);

@@ -47,6 +47,7 @@ enum FlagSlot : int {
   kFlagTicket2 = 4,   // ticket of the large-layer pass
   kFlagBigCount = 5,  // layers of the large-layer pass
   kFlagOrdered = 6,   // non-empty layers in the size order
+  kFlagTicketScatter = 7,
   kFlagCount = 8
 };
 
