@@ -437,8 +437,10 @@ void chunk_events(int32_t E, const int64_t* off, int nch, int32_t* cev) {
   }
 }
 
-int grid_for(int64_t n) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16));
+int grid_for(int64_t n, int device) {
+  int sms = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, sms * 16));
 }
 
 }  // namespace
@@ -550,7 +552,7 @@ int clue_bridge_build(clue_handle* hh, const clue_bridge_params* p, int32_t E, c
                                                                      clusterIndex, acc, seed_of, flags);
     if ((e = cudaGetLastError())) return cuda_error(e, "k_bridge_accumulate");
     if (C > 0)
-      clue::k_bridge_finalize<<<clue::grid_for(C), 256, 0, s>>>(C, acc, seed_of, x, y, layer,
+      clue::k_bridge_finalize<<<clue::grid_for(C, h->device), 256, 0, s>>>(C, acc, seed_of, x, y, layer,
                                                                  d_lz, p->n_layers, p->radius, p->isSilicon, *out, flags);
     if ((e = cudaGetLastError())) return cuda_error(e, "k_bridge_finalize");
     if ((e = cudaMemcpyAsync(h->flags_host.p, flags, 4 * clue::kFlagCount, cudaMemcpyDeviceToHost, s)) ||
