@@ -1612,15 +1612,21 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
     big.threads = tt.big_threads;
     big.layer_capacity = tt.big_capacity;
     if (two_class && b.use_order) {
-      // The large layers on this stream, the others from the same point on the
-      // side stream: the CTAs of the pass over the small layers start as those
-      // of the large pass run out of layers, instead of after the last one has
-      // ended, and the large layers start first, not last (48 uneven events 295
-      // -> 261 us; 200 HGCAL events, all of whose layers are large, 5.61 -> 5.58 ms).
-      // With up to three layers per CTA one after the other, large layers first: side
-      // by side their few long layers share SMs to the end (8 events 154 against
-      // 120 us, 12: 159 / 132, 16: 142 / 134; but 24: 178 / 210, 48: 257 / 280).
-      if (n_items <= 3 * grid) side = nullptr;
+      // The large layers first, so that they do not start last.  In a captured
+      // run the others go beside them, from the same point on the side stream: their
+      // CTAs start as the large pass runs out of layers, instead of after its last
+      // one has ended (48 uneven events replayed 289 -> 264 us, 380: 1.95 -> 1.91 ms).
+      // With up to three layers per CTA one after the other: side by side their few
+      // long layers share SMs to the end (8 events 154 against 120 us, 12: 159 / 132,
+      // 16: 142 / 134; but 24: 178 / 210).  Direct launches go one after the other
+      // as well: there the side stream's pass often took the SMs first and the large
+      // layers came last (48 events 342 against 299 us; 65 of which two layers hold a
+      // third 2.46 against 1.36 ms; 380 even ones 1.94 against 1.95).
+      if (side) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if ((err = cudaStreamIsCapturing(s, &capture)) != cudaSuccess) return err;
+        if (capture == cudaStreamCaptureStatusNone || n_items <= 3 * grid) side = nullptr;
+      }
       const LaunchKind kind = side ? kOrdinary : kDependent;
       Batch2D large = b;
       large.cursor = b.order;  // the list that the large-layer pass drains
@@ -1633,6 +1639,7 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
       if (err == cudaSuccess && side) err = cudaEventRecord(side->join, s2);
       if (err == cudaSuccess && side) err = cudaStreamWaitEvent(s, side->join, 0);
     } else {
+      side = nullptr;
       err = launch_layers_any(tt.threads, b, p, tt.layer_capacity, max_m, 0, grid, s, kDependent);
       if (err == cudaSuccess && two_class)
         err = launch_layers_any(big.threads, b, p, big.layer_capacity, INT_MAX, 1, layer_grid(big, n_items), s, kDependent);
@@ -1648,7 +1655,7 @@ cudaError_t launch_clue2d(const Batch2D& batch, const Params2D& p, const Tuning2
     const bool wide = !b.seed_bits || nc >= 24 * (int64_t)b.n_events;
     auto* k = !b.seed_bits ? k_seed_chunk_scan<false, 1024> : wide ? k_seed_chunk_scan<true, 1024> : k_seed_chunk_scan<true, 256>;
     const int threads = wide ? 1024 : 256;
-    if (two_class && b.use_order) {  // behind the join of the two passes
+    if (side) {  // behind the join of the two passes
       k<<<b.n_events, threads, 0, s>>>(b);
       err = cudaGetLastError();
     } else {

@@ -139,7 +139,7 @@ cudaError_t prepare_clue2d_kernels(int device);
 bool layers_ordered(const Tuning2D& t, int n_items);
 
 // A second stream and two events, for the pass over the small layers of an
-// ordered batch (without them it follows the pass over the large ones).
+// ordered batch that is captured (else it follows the pass over the large ones).
 struct SideStream {
   cudaStream_t stream = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;

@@ -833,8 +833,6 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
       return cuda_error(e, "cudaEventCreate");
     }
   }
-  for (int i = 0; i < S; ++i)  // before any copy into or out of the caller's arrays is queued
-    if ((rc = h->ensure_side(cut[i + 1] - cut[i]))) return rc;
   cudaEvent_t* h2d = h->pipe_events;
   cudaEvent_t* comp = h->pipe_events + kPipeSlots;
   cudaEvent_t* d2h = h->pipe_events + 2 * kPipeSlots;
@@ -880,7 +878,7 @@ int run_2d_pipelined(Handle* h, const Run2D& r) {
     if ((e = cudaStreamWaitEvent(cs, h2d[k], 0)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(cs, d2h[k], 0)) != cudaSuccess)
       return cuda_error(e, "sub-batch set-up");
-    if ((e = launch_clue2d(b, h->p2d, h->tuning, cs, nullptr, &kernels, h->side_stream())) != cudaSuccess)
+    if ((e = launch_clue2d(b, h->p2d, h->tuning, cs, nullptr, &kernels)) != cudaSuccess)
       return cuda_error(e, "launching CLUE kernels");
     if ((e = cudaEventRecord(comp[k], cs)) != cudaSuccess) return cuda_error(e, "cudaEventRecord");
     const clue_outputs* o = r.out;
