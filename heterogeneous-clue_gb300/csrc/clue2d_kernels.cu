@@ -506,8 +506,10 @@ __device__ void process_layer(const Params2D& P, const LayerStore<TT, QT>& S, co
   // threshold at 512).  So do layers in HBM scratch, in the tiles' order:
   // neighbouring queries read the same lines, which the order by count scatters
   // (one event of 200,000 points, 43,000 on a layer, dc 5.5 cm: 3.27 -> 2.28 ms,
-  // and 2.96 with finer buckets; 600,000 points, 6,000 to a layer: 152 -> 134 us).
-  if (m > 256 && sizeof(TT) == 2) {
+  // and 2.96 with finer buckets; 600,000 points, 6,000 to a layer: 152 -> 134 us),
+  // unless the boxes hold one tile or four (two events, 47,000 points on a layer
+  // each, boxes of 1.8 cm: 3.58 ms, 3.84 without the order).
+  if (m > 256 && (sizeof(TT) == 2 || P.dm < 2.5f)) {
     order_queries<NT>(S, m, P.dm, s_bins);
   } else {
     for (int i = tid; i < m; i += NT) S.qord[i] = (QT)i;

@@ -36,3 +36,19 @@ def test_layers_over_the_capacity(cuda_lib, events, sizes, prm, shuffled):
     want = oracle.clue2d_batch(off, x, y, layer, w, *prm, n_threads=8)
     assert_bitexact(got, want)
     assert_bitexact(small, want)
+
+
+@pytest.mark.parametrize("events", [1, 3, 12])
+@pytest.mark.parametrize("n,rhoc", [(4200, 1.0), (20000, 1.0), (9000, 1e9)])
+def test_long_chains(cuda_lib, events, n, rhoc):
+    """Points on a line whose density rises along it: chains of thousands of steps,
+    which end at a seed or at an outlier."""
+    x = np.tile(np.linspace(-245, 245, n), events).astype(np.float32)
+    y = np.zeros(n * events, np.float32)
+    w = np.tile(np.linspace(1, 40, n), events).astype(np.float32)
+    layer = np.full(n * events, 3, np.int32)
+    off = np.arange(events + 1, dtype=np.int64) * n
+    algo = C.Clusterizer(1.3, rhoc, 2.0)
+    got = algo.run_batch(off, x, y, layer, w)
+    algo.close()
+    assert_bitexact(got, oracle.clue2d_batch(off, x, y, layer, w, 1.3, rhoc, 2.0, n_threads=8))
