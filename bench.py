@@ -57,7 +57,7 @@ K_LAYERS_DRAM_BYTES_PER_POINT = 24.67
 # peak (4 schedulers x 1 instruction per cycle) is the bound that applies.
 K_LAYERS_WARP_INST_PER_POINT = 85.54
 # Where the two figures come from (reported with them in the JSON line).
-K_LAYERS_CAPTURE = {"commit": "9fb9e81", "summary": "profiles/k_layers_uneven256.md",
+K_LAYERS_CAPTURE = {"commit": "9fb9e81", "tool": "ncu: DRAM bytes and warp instructions per launch",
                     "workload": "256-event uneven batch, 13,628,373 points, both passes"}
 
 

@@ -385,8 +385,9 @@ struct NhBest {
       k = pos;
     }
   }
+  __device__ __forceinline__ bool near() const { return near(d2, prev); }
   // sqrt_rn(a) < sqrt_rn(b) whenever a * 1.00002f < b
-  __device__ __forceinline__ bool near() const { return !(__fmul_rn(d2, 1.00002f) < prev); }
+  static __device__ __forceinline__ bool near(float d2, float prev) { return !(__fmul_rn(d2, 1.00002f) < prev); }
 };
 
 // One (event, layer) item through every stage.  next_item: in thread 0, the
@@ -754,7 +755,7 @@ __device__ __forceinline__ void tiny_layer(const Params2D& P, unsigned char* ws,
     const int q = lane + 32 * j;
     if (q >= m) continue;
     float best_s = best[j] >= 0 ? __fsqrt_rn(d2[j]) : FLT_MAX;
-    if (best[j] >= 0 && !(__fmul_rn(d2[j], 1.00002f) < prev[j])) {
+    if (best[j] >= 0 && NhBest::near(d2[j], prev[j])) {
       best_s = FLT_MAX;
       best[j] = -1;
       for (int k = 0; k < m; ++k) {
@@ -1213,6 +1214,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_layers(Batch2D b, Params2D P,
       if (threadIdx.x == 0) big_list[atomicAdd(&b.flags[kFlagBigCount], 1)] = item;
       continue;
     }
+    // (layer_io() written out: with the call 60 HGCAL events took 1.669 ms against 1.657)
     const int e = item / kLayers;
     const int64_t es = b.offsets[e];
     const int start = b.lstart[item];

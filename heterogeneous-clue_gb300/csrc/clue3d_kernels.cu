@@ -173,7 +173,7 @@ __global__ void k3_key(Batch3D b, Params3D P) {
       k = l * kBins + pb + eta_bin(b.eta[i], P) * kPhiBins;
     }
     b.key[i] = k;
-    if (k < 0) b.seed[i] = -1;  // not searched: k3_finish makes it a root of its own
+    if (k < 0) b.seed[i] = -1;  // not searched: k3_rank makes it a root of its own
     row = row_of(k, b.n_rows);
   }
   const int gkey = row >= 0 ? e * b.n_rows + row : -1;
@@ -965,7 +965,8 @@ __global__ void k3_label(Batch3D b) {
 }  // namespace
 
 cudaError_t prepare_clue3d_kernels() {
-  // more than the 48 KB a kernel may use without asking
+  // also loads the kernels' code, so that no launch has any to load (the staging
+  // itself, 44 KB, is within what a kernel may use without asking)
   for (auto* k : {k3_search<true, kWhole>, k3_search<true, kInParts>, k3_search<true, kGlobal>, k3_search<false, kWhole>,
                   k3_search<false, kInParts>, k3_search<false, kGlobal>}) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem);

@@ -355,7 +355,7 @@ __device__ __forceinline__ Ff ff_atan(Ff q) {
 // single-precision rate: the double form bounded the kernel, 200 HGCAL events
 // 0.271 ms, this 0.041 ms).  Sums of two floats give each field to 2^-40 and
 // better; where that leaves its rounding to float in doubt (one cluster in
-// some hundreds) or a value is out of the forms' range, returns false and the
+// some 1,600) or a value is out of the forms' range, returns false and the
 // double form decides, so the results are the double form's.
 __device__ __forceinline__ bool cluster_fast(long long sw, long long swx, long long swy, float z, ClusterFields* o) {
   constexpr long long kMost = 1ll << 46;

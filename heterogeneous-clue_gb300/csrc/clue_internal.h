@@ -177,7 +177,7 @@ struct Batch3D {
   int32_t n_events = 0;
   int64_t n_points = 0;
   int64_t max_event = 0;  // clusters of the largest event
-  int32_t n_rows = 0;  // rows (layer, eta) per event: n_layers * 34 + 1
+  int32_t n_rows = 0;  // rows (layer, eta) per event: n_layers * 34, the one behind them and that of rejected clusters
   // page-locked host memory the kernels read and write: the offset and block
   // tables (copied to table_dst), the trackster counts and status words
   // (nullptr: none), and of a small host run its inputs (n_in16 x 16 bytes,

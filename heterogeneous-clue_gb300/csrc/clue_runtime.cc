@@ -727,8 +727,8 @@ int run_2d_plain(Handle* h, const Run2D& r) {
     if (any_error) return set_error(CLUE_EINVAL, "a point has a layer outside [0, %d)", kLayers);
     return CLUE_OK;
   }
-  // device mode: the error word accumulates over the events (launch_clue2d
-  // never clears it) and is read back at clue_synchronize.
+  // device mode: the error word accumulates over the events (clear_error = 0
+  // keeps k_init from clearing it) and is read back at clue_synchronize.
   e = cudaMemcpyAsync(h->flags_host.p, h->arena.ptr(S_FLAGS), 4 * kFlagCount, cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return cuda_error(e, "D2H status");
   h->last_run.d2h_bytes = 4 * kFlagCount;
