@@ -379,6 +379,7 @@ struct Run2D {
   const float* w;
   const clue_outputs* out;
   int flags;
+  bool in_one = false, out_one = false;  // host inputs / outputs that move in one copy each
 };
 
 // Whether none of a run's arrays is pageable.
@@ -407,13 +408,8 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
   cudaStream_t s = h->stream;
   cudaError_t e;
   const size_t n4 = 4 * (size_t)r.N;
-  // back-to-back host arrays (a server's staging is laid out so) move in one copy
-  const bool known = r.flags & kAsyncHostIO, copies = host_io && !b.host_in;
-  const bool in_one = known || (copies && one_copy({r.x, r.y, r.layer, r.w}, n4));
-  const bool out_one = known || (copies && one_copy({r.out->rho, r.out->delta, r.out->nearestHigher, r.out->isSeed,
-                                                     r.out->clusterIndex}, n4));
-  if (copies) {
-    if (in_one) {
+  if (host_io && !b.host_in) {
+    if (r.in_one) {
       if ((e = cudaMemcpyAsync((void*)b.x, r.x, 4 * n4, cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return cuda_error(e, "H2D points");
     } else if ((e = cudaMemcpyAsync((void*)b.x, r.x, n4, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
@@ -427,7 +423,7 @@ int enqueue_2d(Handle* h, const Run2D& r, Batch2D& b, bool host_io, cudaEvent_t*
   if (e != cudaSuccess) return cuda_error(e, "launching CLUE kernels");
   if (host_io && !b.host_out) {
     const clue_outputs* o = r.out;
-    if (out_one) {
+    if (r.out_one) {
       if ((e = cudaMemcpyAsync(o->rho, b.rho, 5 * n4, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return cuda_error(e, "D2H outputs");
     } else if ((e = cudaMemcpyAsync(o->rho, b.rho, n4, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
@@ -556,6 +552,14 @@ int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nul
     b.host_out = r.out->rho;
   }
 
+  if (host_io && !staged) {
+    // back-to-back arrays (a server's staging is laid out so)
+    const size_t n4 = 4 * (size_t)r.N;
+    const bool known = r.flags & kAsyncHostIO;
+    r.in_one = known || one_copy({r.x, r.y, r.layer, r.w}, n4);
+    r.out_one = known || one_copy({r.out->rho, r.out->delta, r.out->nearestHigher, r.out->isSeed, r.out->clusterIndex}, n4);
+  }
+
   bool use_graph = !(r.flags & CLUE_NO_GRAPH) && !stage_events;
   if (use_graph && host_io && !staged) {
     // graph memcpy nodes need page-locked host memory
@@ -564,7 +568,8 @@ int run_2d_batched(Handle* h, const Run2D& r_in, cudaEvent_t* stage_events = nul
   cudaError_t e;
   int64_t kernels = 0;
   if (use_graph) {
-    GraphKey key{r.E, r.N, nchunks, h->arena.generation(), r.flags, priority_of(h->stream), h->tuning.threads,
+    GraphKey key{r.E, r.N, nchunks, h->arena.generation(), r.flags, priority_of(h->stream),
+                 (r.in_one ? 1 : 0) | (r.out_one ? 2 : 0), h->tuning.threads,
                  h->tuning.layer_capacity, h->tuning.ctas_per_sm,
                  h->tuning.big_threads, h->tuning.big_capacity,
                  h->tuning.work_tile_cm, h->p2d.dc, h->p2d.rhoc, h->p2d.odf,

@@ -74,13 +74,14 @@ struct GraphKey {
   uint64_t arena_gen = 0;   // and so are the addresses of every arena buffer
   int flags = 0;
   int priority = 0;         // of the captured stream: kernel nodes keep it
+  int one_copy = 0;         // inputs, outputs in one copy each
   int threads = 0, cap = 0, ctas = 0, big_threads = 0, big_cap = 0;
   float work_tile = 0.f;
   float dc = 0.f, rhoc = 0.f, odf = 0.f;
   const void* ptrs[14] = {};
   bool operator==(const GraphKey& o) const {
     if (E != o.E || N != o.N || nchunks != o.nchunks || arena_gen != o.arena_gen || flags != o.flags ||
-        priority != o.priority ||
+        priority != o.priority || one_copy != o.one_copy ||
         threads != o.threads || cap != o.cap || ctas != o.ctas ||
         big_threads != o.big_threads || big_cap != o.big_cap ||
         work_tile != o.work_tile || dc != o.dc || rhoc != o.rhoc || odf != o.odf)
